@@ -16,6 +16,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <utility>
 
 #include "device_bsdf.cuh"
 #include "device_medium.cuh"
@@ -49,6 +50,8 @@ struct __align__(16) PathScalars {
 };
 static_assert(sizeof(PathScalars) == 32, "one sector per path");
 
+constexpr int kCtrStride = 14;   // words of a bounce's counter block, see kCtr*
+
 struct WaveState {
     float4* ray;         // [N][2]: origin xyz + tmin, direction xyz + tmax (one sector per path)
     float4* hit;         // t, b1, b2, prim bits
@@ -63,7 +66,43 @@ struct WaveState {
     uint32_t* counters;    // [kCtrStride * (maxDepth + 2)], see kCtr*
     unsigned long long* stats;  // 0 extension rays, 1 shadow rays, 2 dropped samples
     uint32_t N;
+    uint32_t hostTag;           // of the wave (BounceCounts)
+    unsigned long long* hostCounts;   // [bounce]: hostTag << 32 | paths, for the host; null where it does not look
 };
+
+// ---------------------------------------------------------------------------
+// Launch order inside a wave (programmatic dependent launch)
+//
+// A kernel of a wave starts in one of two ways.  One that needs its
+// predecessor's results ("after") is put on the SMs while the predecessor
+// drains and waits at its first instruction until it has completed.  One that
+// needs nothing of its predecessor, only what was complete when that
+// predecessor started ("beside": the shadow rays of the last bounce beside the
+// extension rays of the next, the shading kernels of a bounce beside each
+// other), starts as soon as all blocks of the predecessor have, and waits for
+// it at its end instead, so that "this kernel has completed" always
+// includes everything launched before it.  Every kernel lets its successor
+// start once its own wait at the start is over.  Few-path bounces cost the
+// latency of their slowest thread: side by side they cost the longer of two
+// latencies and not the sum (64 x 64 x 1 box: 526 to 392 us, the 176k-triangle
+// terrain at 512 x 512 x 4: 3.33 to 2.35 ms, every kind of BSDF at 333 x 187 x
+// 24: 3.36 to 2.17 ms).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void waveBegin(bool beside) {
+    if (!beside) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// One thread holds the kernel's completion for the predecessor's.
+__device__ __forceinline__ void waveEnd(bool beside) {
+    if (beside && blockIdx.x == 0 && threadIdx.x == 0) asm volatile("griddepcontrol.wait;");
+}
+// The host's view of a bounce's size, written as the bounce starts.
+__device__ __forceinline__ void tellHost(const WaveState &ws, const uint32_t* rowCounters, uint32_t n) {
+    if (ws.hostCounts == nullptr || blockIdx.x != 0 || threadIdx.x != 0) return;
+    const uint32_t bounce = (uint32_t)(rowCounters - ws.counters) / kCtrStride;
+    *(volatile unsigned long long*)(ws.hostCounts + bounce) = ((unsigned long long)ws.hostTag << 32) | n;
+    __threadfence_system();
+}
 
 // The reference's renderers sample the sensor in whole 8x8 tiles
 // (ImageSensor.cpp:13-14, :42-43; PTRenderer.cpp:104-110), also where a tile
@@ -159,13 +198,13 @@ constexpr int kClassMiss = 5;
 constexpr int kClassMedium = 6;       // volumetric: a scattering point in the medium
 constexpr int kQueueMedShadow = 7;    // volumetric: unoccluded shadow rays waiting for their transmittance
 constexpr int kNumClassQueues = 8;
-constexpr int kCtrStride = 13;
 constexpr int kCtrExt = 7;
 constexpr int kCtrShadow = 8;
 constexpr int kCtrMedShadow = 9;
 constexpr int kCtrMedTake = 10;
 constexpr int kCtrExtTake = 11;
 constexpr int kCtrShadowTake = 12;
+constexpr int kCtrTailRow = 13;       // row 0 only: 1 + the bounce that kTail starts at, 0 while there is none
 // hit.w of a path whose ray stopped at a collision in the medium (hit.x = its
 // distance, hit.y = 1 inside the density grid's unit cube)
 constexpr uint32_t kMediumHit = 0xfffffffeu;
@@ -200,9 +239,13 @@ __device__ __forceinline__ uint64_t loadKey(const WaveState &ws, uint32_t p) {
 template <bool MULTI>
 __global__ void kRaygen(DevScene scArg, WaveState ws, const __grid_constant__ WaveParams wpArg,
                         const WaveParams* __restrict__ wpDev, const DevScene* __restrict__ scenes,
-                        bool initAlpha) {
+                        bool initAlpha, uint32_t tailPaths) {
     const WaveParams &wp = wpDev ? *wpDev : wpArg;
-    if (blockIdx.x == 0 && threadIdx.x == 0) ws.counters[kCtrExt] = wp.numPaths;
+    waveBegin(false);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        ws.counters[kCtrExt] = wp.numPaths;
+        if (wp.numPaths <= tailPaths) ws.counters[kCtrTailRow] = 1;
+    }
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < wp.numPaths; p += gridDim.x * blockDim.x) {
         uint32_t k = 0;
         while (k + 1 < wp.numSegments && p >= wp.seg[k + 1].pathBegin) ++k;
@@ -342,9 +385,11 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadow(DevScene
                                                                       const uint32_t* __restrict__ count,
                                                                       uint32_t* cursor,
                                                                       const DevScene* __restrict__ scenes) {
+    waveBegin(true);
     const uint32_t n = *count;
 #if SLRGPU_TRACE_REFILL
-    if (scArg.watertight) shadowRefill<MULTI, true>(scArg, ws, queue, n, cursor, scenes);
+    if (n == 0) {
+    } else if (scArg.watertight) shadowRefill<MULTI, true>(scArg, ws, queue, n, cursor, scenes);
     else shadowRefill<MULTI, false>(scArg, ws, queue, n, cursor, scenes);
 #else
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -359,6 +404,7 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadow(DevScene
     }
 #endif
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ws.stats[1], (unsigned long long)n);
+    waveEnd(true);
 }
 
 // ---------------------------------------------------------------------------
@@ -455,8 +501,15 @@ template <bool MULTI>
 __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kExtendSort(DevScene scArg, WaveState ws,
                                                                           const uint32_t* __restrict__ queue,
                             const uint32_t* __restrict__ count, uint32_t* classCounts, uint32_t* cursor,
-                            uint32_t maxDepth, const DevScene* __restrict__ scenes) {
+                            uint32_t maxDepth, uint32_t tailPaths, const DevScene* __restrict__ scenes) {
+    waveBegin(false);
     const uint32_t n = *count;
+    tellHost(ws, classCounts, n);
+    if (n <= tailPaths) {   // kTail's (or no paths)
+        if (n != 0 && blockIdx.x == 0 && threadIdx.x == 0)
+            ws.counters[kCtrTailRow] = 1 + (uint32_t)(classCounts - ws.counters) / kCtrStride;
+        return;
+    }
 #if SLRGPU_TRACE_REFILL
     if (scArg.watertight) extendRefill<MULTI, true>(scArg, ws, queue, n, cursor, classCounts, scenes, maxDepth);
     else extendRefill<MULTI, false>(scArg, ws, queue, n, cursor, classCounts, scenes, maxDepth);
@@ -487,7 +540,10 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kExtend(DevScene
                                                                       const uint32_t* __restrict__ queue,
                                                                       const uint32_t* __restrict__ count,
                                                                       uint32_t* cursor) {
+    waveBegin(false);
     const uint32_t n = *count;
+    tellHost(ws, count, n);
+    if (n == 0) return;
 #if SLRGPU_TRACE_REFILL
     if (sc.watertight) extendRefill<false, true, false>(sc, ws, queue, n, cursor, nullptr, nullptr);
     else extendRefill<false, false, false>(sc, ws, queue, n, cursor, nullptr, nullptr);
@@ -506,40 +562,45 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kExtend(DevScene
 // Paths whose ray left the scene: environment emission (with MIS after a
 // non-delta bounce), then the path ends (PTRenderer.cpp:150-152, :234-263).
 template <bool MULTI>
-__global__ void kShadeMiss(DevScene scArg, WaveState ws, const uint32_t* __restrict__ queue,
-                           const uint32_t* __restrict__ count, const DevScene* __restrict__ scenes) {
-    const uint32_t n = *count;
-    if (!MULTI && !scArg.envPresent) return;
+__device__ __forceinline__ void shadeMiss(const DevScene &scArg, const WaveState &ws, uint32_t p,
+                                          const DevScene* __restrict__ scenes) {
     const float twoPi = 6.28318530717958647692f;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t p = queue[i];
-        const uint32_t info = ws.ps[p].info;
-        const DevScene &sc = pathScene<MULTI>(scArg, scenes, info);
-        if (MULTI && !sc.envPresent) continue;     // no environment: the path just ends
-        const uint32_t depth = info >> kInfoDepthShift;
-        const bool prevDelta = (info & kInfoPrevDelta) != 0;
-        const float wlOff = ws.ps[p].wlOffset;
-        const OffsetLambdas lambdas{wlOff};
-        float4 rd = ws.ray[2 * (size_t)p + 1];
-        V3 dir = V3{rd.x, rd.y, rd.z};
-        float theta, phi;
-        toPolarYUp(dir, &theta, &phi);
-        Spec Le;
-        envRadiance(sc, phi / twoPi, theta / kPiF, lambdas, Le);
-        float mis = 1.0f;
-        if (depth > 0 && !prevDelta) {
-            float lightProb = sc.envImportance / (sc.surfImportance + sc.envImportance);
-            float lightPdf = lightProb * envAreaPdf(sc, phi, theta) * 1.0f / absDot(dir, -dir);
-            float bp = ws.ps[p].prevPdf;
-            mis = (bp * bp) / (lightPdf * lightPdf + bp * bp);
-        }
-        Spec a;
-        if (depth == 0) a = specConst(1.0f);
-        else loadSpec(ws.alpha, p, a);
-#pragma unroll
-        for (int k = 0; k < kNumLambda; ++k) a.v[k] = a.v[k] * Le.v[k] * mis;
-        addSpec(ws.L, p, a);
+    const uint32_t info = ws.ps[p].info;
+    const DevScene &sc = pathScene<MULTI>(scArg, scenes, info);
+    if (!sc.envPresent) return;     // no environment: the path just ends
+    const uint32_t depth = info >> kInfoDepthShift;
+    const bool prevDelta = (info & kInfoPrevDelta) != 0;
+    const float wlOff = ws.ps[p].wlOffset;
+    const OffsetLambdas lambdas{wlOff};
+    float4 rd = ws.ray[2 * (size_t)p + 1];
+    V3 dir = V3{rd.x, rd.y, rd.z};
+    float theta, phi;
+    toPolarYUp(dir, &theta, &phi);
+    Spec Le;
+    envRadiance(sc, phi / twoPi, theta / kPiF, lambdas, Le);
+    float mis = 1.0f;
+    if (depth > 0 && !prevDelta) {
+        float lightProb = sc.envImportance / (sc.surfImportance + sc.envImportance);
+        float lightPdf = lightProb * envAreaPdf(sc, phi, theta) * 1.0f / absDot(dir, -dir);
+        float bp = ws.ps[p].prevPdf;
+        mis = (bp * bp) / (lightPdf * lightPdf + bp * bp);
     }
+    Spec a;
+    if (depth == 0) a = specConst(1.0f);
+    else loadSpec(ws.alpha, p, a);
+#pragma unroll
+    for (int k = 0; k < kNumLambda; ++k) a.v[k] = a.v[k] * Le.v[k] * mis;
+    addSpec(ws.L, p, a);
+}
+
+template <bool MULTI>
+__global__ void kShadeMiss(DevScene scArg, WaveState ws, const uint32_t* __restrict__ queue,
+                           const uint32_t* __restrict__ count, const DevScene* __restrict__ scenes, bool beside) {
+    waveBegin(beside);
+    const uint32_t n = *count;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        shadeMiss<MULTI>(scArg, ws, queue[i], scenes);
+    waveEnd(beside);
 }
 
 // Resident blocks per SM the shading kernels are compiled for (register cap
@@ -575,242 +636,377 @@ __device__ __forceinline__ SurfPoint loadSurfShared(const float* s) {
 #ifndef SLRGPU_SHADE_DIELECTRIC_MIN_BLOCKS
 #define SLRGPU_SHADE_DIELECTRIC_MIN_BLOCKS SLRGPU_SHADE_MIN_BLOCKS
 #endif
+// Shades path p's vertex with material kind K: emission, roulette, next-event
+// estimation and BSDF sampling.  *shadow: the path has a shadow ray with a
+// stored contribution; *extend: it goes on along a new ray.  sAlpha, sSurf:
+// the block's shared arrays (blocks of 256 threads).
+template <int K, bool MULTI>
+__device__ __forceinline__ void shadeVertex(const DevScene &scArg, const WaveState &ws, uint32_t p, uint32_t maxDepth,
+                                            const DevScene* __restrict__ scenes, float* sAlpha, float* sSurf,
+                                            bool &extend, bool &shadow) {
+    const float inf = __int_as_float(0x7f800000);
+    const float twoPi = 6.28318530717958647692f;
+#if SLRGPU_SHADE_SMEM_ALPHA
+    // the path's throughput in shared memory ([wavelength][thread]), not in
+    // registers, through light and BSDF sampling
+#define SLRGPU_ALPHA(k) sAlpha[(k) * 256 + threadIdx.x]
+#endif
+    uint32_t info = ws.ps[p].info;
+    const DevScene &sc = pathScene<MULTI>(scArg, scenes, info);
+    const uint32_t sceneBits = info & kInfoSceneMask;
+    const int sel = (int)(info & kInfoSelMask);
+    bool wlSelected = (info & kInfoWlSelected) != 0;
+    const bool prevDelta = (info & kInfoPrevDelta) != 0;
+    uint32_t depth = info >> kInfoDepthShift;
+    const float wlOff = ws.ps[p].wlOffset;
+    const OffsetLambdas lambdas{wlOff};
+    Rng rng{loadKey(ws, p), ws.ps[p].rngCounter, sc.rngTape};
+    float4 ro = ws.ray[2 * (size_t)p], rd = ws.ray[2 * (size_t)p + 1];
+    V3 org = V3{ro.x, ro.y, ro.z}, dir = V3{rd.x, rd.y, rd.z};
+    float4 hv = ws.hit[p];
+    const DevPrim pr = sc.prims[__float_as_uint(hv.w)];
+#if SLRGPU_SHADE_SMEM_ALPHA
+    {
+        Spec a0;
+        if (depth == 0) a0 = specConst(1.0f);
+        else loadSpec(ws.alpha, p, a0);
+#pragma unroll
+        for (int k = 0; k < kNumLambda; ++k) SLRGPU_ALPHA(k) = a0.v[k];
+    }
+#else
+    Spec alpha;
+    if (depth == 0) alpha = specConst(1.0f);
+    else loadSpec(ws.alpha, p, alpha);
+#define SLRGPU_ALPHA(k) alpha.v[k]
+#endif
+    bool alive = true;
+    SurfPoint sp;
+    surfacePoint(sc, pr, org, dir, hv.x, hv.y, hv.z, sp);
+    const DevMaterial mat = sc.materials[pr.material];
+    V3 dirOut = sp.frame.toLocal(-dir);
+    // Emission on hit (PTRenderer.cpp:162-166, :240-263).
+    if (mat.emit >= 0) {
+        Spec M;
+        evalSpectrum(sc, mat.emit, lambdas, M);
+        float edf = dirOut.z > 0.0f ? kInvPiF : 0.0f;
+        float mis = 1.0f;
+        if (depth > 0 && !prevDelta) {
+            float lightProb = (sc.surfImportance / (sc.surfImportance + sc.envImportance)) * sc.lightPMF[0];
+            float dist2 = sqLength(sp.p - org);
+            float lightPdf = lightProb * pr.invArea * dist2 / absDot(dir, sp.gn);
+            float bp = ws.ps[p].prevPdf;
+            mis = (bp * bp) / (lightPdf * lightPdf + bp * bp);
+        }
+        Spec add;
+#pragma unroll
+        for (int k = 0; k < kNumLambda; ++k) add.v[k] = SLRGPU_ALPHA(k) * (M.v[k] * edf) * mis;
+        addSpec(ws.L, p, add);
+    }
+    // Russian roulette (PTRenderer.cpp:266-272); a material that does
+    // not emit had its draw at the hit (rouletteAtHit), and the path
+    // is here because it continued.
+    if (depth > 0) {
+        Spec a1;
+#pragma unroll
+        for (int k = 0; k < kNumLambda; ++k) a1.v[k] = SLRGPU_ALPHA(k);
+        float cp = fminf(importance(a1, sel) / ws.ps[p].initY, 1.0f);
+        if ((SLRGPU_EARLY_ROULETTE && mat.emit < 0) || rng.next() < cp) {
+            float r = 1.0f / cp;
+#pragma unroll
+            for (int k = 0; k < kNumLambda; ++k) SLRGPU_ALPHA(k) *= r;
+        } else {
+            alive = false;
+        }
+    }
+    if (alive) {
+        ++depth;
+        if (depth > maxDepth) alive = false;
+    }
+    if (alive) {
+        Bsdf B;
+        makeBsdfK<K>(sc, mat, lambdas, wlSelected, B);
+        BsdfQuery q{dirOut, sp.frame.toLocal(sp.gn), sel};
+#if SLRGPU_SHADE_SMEM_SP
+        storeSurfShared(sSurf, sp);
+#define SLRGPU_SP() loadSurfShared(sSurf)
+#else
+#define SLRGPU_SP() sp
+#endif
+        // Next-event estimation (PTRenderer.cpp:179-218).
+        if (bsdfHasNonDelta(K) && (sc.numLights > 0 || sc.envPresent)) {
+            const SurfPoint spN = SLRGPU_SP();
+            float lightProb;
+            int li = selectLight(sc, rng.next(), &lightProb);
+            float lu0 = rng.next(), lu1 = rng.next();
+            V3 lp, lgn;
+            Spec M;
+            float areaPdf, edfVal, dist2;
+            bool atInf = false;
+            V3 shadowDir;
+            if (li >= 0) {
+                const DevPrim lpr = sc.prims[sc.lightPrims[li]];
+                float su = sqrtf(lu0);
+                float b0 = 1.0f - su, b1 = lu1 * su, b2 = 1.0f - b0 - b1;
+                float4 p0 = sc.vpos[lpr.v0], p1 = sc.vpos[lpr.v1], p2 = sc.vpos[lpr.v2];
+                lp = rn_bary(b0, V3{p0.x, p0.y, p0.z}, b1, V3{p1.x, p1.y, p1.z}, b2, V3{p2.x, p2.y, p2.z});
+                float4 n0 = sc.vnrm[lpr.v0], n1 = sc.vnrm[lpr.v1], n2 = sc.vnrm[lpr.v2];
+                V3 lz = normalize(b0 * V3{n0.x, n0.y, n0.z} + b1 * V3{n1.x, n1.y, n1.z} + b2 * V3{n2.x, n2.y, n2.z});
+                lgn = V3{lpr.ngx, lpr.ngy, lpr.ngz};
+                areaPdf = lpr.invArea;
+                evalSpectrum(sc, sc.materials[lpr.material].emit, lambdas, M);
+                V3 diff = lp - spN.p;
+                dist2 = sqLength(diff);
+                shadowDir = diff * (1.0f / sqrtf(dist2));
+                edfVal = dot(lz, -shadowDir) > 0.0f ? kInvPiF : 0.0f;
+            } else {
+                float uvPdf, topPdf;
+                uint32_t row, col;
+                float d1 = sampleAlias(sc.envTopAlias, sc.envTopPDF, sc.envMapH, lu1, &topPdf, &row);
+                float d0 = sampleAlias(sc.envRowAlias + (size_t)row * sc.envMapW,
+                                       sc.envRowPDF + (size_t)row * sc.envMapW, sc.envMapW, lu0, &uvPdf, &col);
+                uvPdf *= topPdf;
+                float phi = d0 * twoPi, theta = d1 * kPiF;
+                float sph, cph, sth, cth;
+                sincosf(phi, &sph, &cph);
+                sincosf(theta, &sth, &cth);
+                lp = V3{-sph * sth, cth, cph * sth};
+                lgn = -lp;
+                atInf = true;
+                areaPdf = uvPdf / (2.0f * kPiF * kPiF * sth);
+                envRadiance(sc, phi / twoPi, theta / kPiF, lambdas, M);
+                edfVal = 1.0f;
+                shadowDir = normalize(lp);
+                dist2 = 1.0f;
+            }
+            float cosShading = absDot(shadowDir, spN.gn);
+            float cosLight = absDot(shadowDir, lgn);
+            if (cosShading * cosLight > 0) {
+                float lightPdf = lightProb * areaPdf;
+                V3 sdl = spN.frame.toLocal(shadowDir);
+                Spec fs;
+                bsdfEval<K>(B, q, sdl, fs);
+                float bsdfPdfV = bsdfPdf<K>(B, q, sdl) * cosLight / dist2;
+                float mis = 1.0f;
+                if (!isinf(areaPdf))
+                    mis = (lightPdf * lightPdf) / (lightPdf * lightPdf + bsdfPdfV * bsdfPdfV);
+                float G = cosShading * cosLight / dist2;
+                float scale = G * mis / lightPdf;
+                Spec c;
+                bool nz = false;
+#pragma unroll
+                for (int k = 0; k < kNumLambda; ++k) {
+                    c.v[k] = ((SLRGPU_ALPHA(k) * (M.v[k] * edfVal)) * fs.v[k]) * scale;
+                    nz |= c.v[k] != 0.0f;
+                }
+                if (nz) {
+                    storeSpec(ws.shContrib, p, c);
+                    float tmax;
+                    V3 sdir;
+                    if (atInf) {
+                        sdir = shadowDir;
+                        tmax = 3.402823466e+38f;
+                    } else {
+                        V3 dd = lp - spN.p;
+                        float dist = length(dd);
+                        sdir = dd * (1.0f / dist);
+                        tmax = dist * (1 - kRayEpsilon);
+                    }
+                    ws.shRay[2 * (size_t)p] = make_float4(spN.p.x, spN.p.y, spN.p.z, kRayEpsilon);
+                    ws.shRay[2 * (size_t)p + 1] = make_float4(sdir.x, sdir.y, sdir.z, tmax);
+                    shadow = true;
+                }
+            }
+        }
+        // BSDF sampling (PTRenderer.cpp:220-236).
+        float uc = rng.next(), u0 = rng.next(), u1 = rng.next();
+        BsdfSample bs;
+        Spec fs;
+        bsdfSample<K>(B, q, uc, u0, u1, &bs, fs);
+        if (bs.pdf == 0.0f || specIsZero(fs)) {
+            alive = false;
+        } else {
+            if ((bs.type & kDirDispersive) && !wlSelected) {
+                bs.pdf /= kNumLambda;
+                wlSelected = true;
+            }
+            float cg = absDot(bs.dir, q.gn);
+            float r = 1.0f / bs.pdf;
+#pragma unroll
+            for (int k = 0; k < kNumLambda; ++k) SLRGPU_ALPHA(k) *= (fs.v[k] * cg) * r;
+            const SurfPoint spS = SLRGPU_SP();
+            V3 nd = spS.frame.fromLocal(bs.dir);
+            ws.ray[2 * (size_t)p] = make_float4(spS.p.x, spS.p.y, spS.p.z, kRayEpsilon);
+            ws.ray[2 * (size_t)p + 1] = make_float4(nd.x, nd.y, nd.z, inf);
+            ws.ps[p].prevPdf = bs.pdf;
+            info = (uint32_t)sel | (wlSelected ? kInfoWlSelected : 0u) |
+                   (dirIsDelta(bs.type) ? kInfoPrevDelta : 0u) | (depth << kInfoDepthShift) | sceneBits;
+            ws.ps[p].info = info;
+            {
+                Spec a2;
+#pragma unroll
+                for (int k = 0; k < kNumLambda; ++k) a2.v[k] = SLRGPU_ALPHA(k);
+                storeSpec(ws.alpha, p, a2);
+            }
+            extend = true;
+        }
+    }
+    ws.ps[p].rngCounter = rng.counter;
+}
+#undef SLRGPU_ALPHA
+#undef SLRGPU_SP
+
 template <int K, bool MULTI>
 __global__ void __launch_bounds__(256, K == kMatGGXScattering ? SLRGPU_SHADE_DIELECTRIC_MIN_BLOCKS
                                                                : SLRGPU_SHADE_MIN_BLOCKS) kShadeSurf(DevScene scArg, WaveState ws, uint32_t maxDepth,
                                                   const uint32_t* __restrict__ inQueue,
                                                   const uint32_t* __restrict__ inCount, uint32_t* outQueue,
                                                   uint32_t* outCount, uint32_t* shQueue, uint32_t* shCount,
-                                                  const DevScene* __restrict__ scenes) {
+                                                  const DevScene* __restrict__ scenes, bool beside) {
+    if (!MULTI) waveBegin(beside);   // waves of several scenes launch in plain order
     const uint32_t n = *inCount;
-    const uint32_t N = ws.N;
-    const float inf = __int_as_float(0x7f800000);
-    const float twoPi = 6.28318530717958647692f;
-#if SLRGPU_SHADE_SMEM_ALPHA
-    // the path's throughput in shared memory ([wavelength][thread]), not in
-    // registers, through light and BSDF sampling
-    __shared__ float sAlpha[kNumLambda * 256];
-#define SLRGPU_ALPHA(k) sAlpha[(k) * 256 + threadIdx.x]
-#endif
-#if SLRGPU_SHADE_SMEM_SP
+    __shared__ float sAlpha[SLRGPU_SHADE_SMEM_ALPHA ? kNumLambda * 256 : 1];
     // the surface point likewise, from the BSDF query to the new ray
-    __shared__ float sSurf[15 * 256];
-#endif
+    __shared__ float sSurf[SLRGPU_SHADE_SMEM_SP ? 15 * 256 : 1];
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
-        bool active = i < n;
+        const bool active = i < n;
         bool extend = false, shadow = false;
-        uint32_t p = active ? inQueue[i] : 0;
-        if (active) {
-            uint32_t info = ws.ps[p].info;
-            const DevScene &sc = pathScene<MULTI>(scArg, scenes, info);
-            const uint32_t sceneBits = info & kInfoSceneMask;
-            const int sel = (int)(info & kInfoSelMask);
-            bool wlSelected = (info & kInfoWlSelected) != 0;
-            const bool prevDelta = (info & kInfoPrevDelta) != 0;
-            uint32_t depth = info >> kInfoDepthShift;
-            const float wlOff = ws.ps[p].wlOffset;
-            const OffsetLambdas lambdas{wlOff};
-            Rng rng{loadKey(ws, p), ws.ps[p].rngCounter, sc.rngTape};
-            float4 ro = ws.ray[2 * (size_t)p], rd = ws.ray[2 * (size_t)p + 1];
-            V3 org = V3{ro.x, ro.y, ro.z}, dir = V3{rd.x, rd.y, rd.z};
-            float4 hv = ws.hit[p];
-            const DevPrim pr = sc.prims[__float_as_uint(hv.w)];
-#if SLRGPU_SHADE_SMEM_ALPHA
-            {
-                Spec a0;
-                if (depth == 0) a0 = specConst(1.0f);
-                else loadSpec(ws.alpha, p, a0);
-#pragma unroll
-                for (int k = 0; k < kNumLambda; ++k) SLRGPU_ALPHA(k) = a0.v[k];
-            }
-#else
-            Spec alpha;
-            if (depth == 0) alpha = specConst(1.0f);
-            else loadSpec(ws.alpha, p, alpha);
-#define SLRGPU_ALPHA(k) alpha.v[k]
-#endif
-            bool alive = true;
-            SurfPoint sp;
-            surfacePoint(sc, pr, org, dir, hv.x, hv.y, hv.z, sp);
-            const DevMaterial mat = sc.materials[pr.material];
-            V3 dirOut = sp.frame.toLocal(-dir);
-            // Emission on hit (PTRenderer.cpp:162-166, :240-263).
-            if (mat.emit >= 0) {
-                Spec M;
-                evalSpectrum(sc, mat.emit, lambdas, M);
-                float edf = dirOut.z > 0.0f ? kInvPiF : 0.0f;
-                float mis = 1.0f;
-                if (depth > 0 && !prevDelta) {
-                    float lightProb = (sc.surfImportance / (sc.surfImportance + sc.envImportance)) * sc.lightPMF[0];
-                    float dist2 = sqLength(sp.p - org);
-                    float lightPdf = lightProb * pr.invArea * dist2 / absDot(dir, sp.gn);
-                    float bp = ws.ps[p].prevPdf;
-                    mis = (bp * bp) / (lightPdf * lightPdf + bp * bp);
-                }
-                Spec add;
-#pragma unroll
-                for (int k = 0; k < kNumLambda; ++k) add.v[k] = SLRGPU_ALPHA(k) * (M.v[k] * edf) * mis;
-                addSpec(ws.L, p, add);
-            }
-            // Russian roulette (PTRenderer.cpp:266-272); a material that does
-            // not emit had its draw at the hit (rouletteAtHit), and the path
-            // is here because it continued.
-            if (depth > 0) {
-                Spec a1;
-#pragma unroll
-                for (int k = 0; k < kNumLambda; ++k) a1.v[k] = SLRGPU_ALPHA(k);
-                float cp = fminf(importance(a1, sel) / ws.ps[p].initY, 1.0f);
-                if ((SLRGPU_EARLY_ROULETTE && mat.emit < 0) || rng.next() < cp) {
-                    float r = 1.0f / cp;
-#pragma unroll
-                    for (int k = 0; k < kNumLambda; ++k) SLRGPU_ALPHA(k) *= r;
-                } else {
-                    alive = false;
-                }
-            }
-            if (alive) {
-                ++depth;
-                if (depth > maxDepth) alive = false;
-            }
-            if (alive) {
-                Bsdf B;
-                makeBsdfK<K>(sc, mat, lambdas, wlSelected, B);
-                BsdfQuery q{dirOut, sp.frame.toLocal(sp.gn), sel};
-#if SLRGPU_SHADE_SMEM_SP
-                storeSurfShared(sSurf, sp);
-#define SLRGPU_SP() loadSurfShared(sSurf)
-#else
-#define SLRGPU_SP() sp
-#endif
-                // Next-event estimation (PTRenderer.cpp:179-218).
-                if (bsdfHasNonDelta(K) && (sc.numLights > 0 || sc.envPresent)) {
-                    const SurfPoint spN = SLRGPU_SP();
-                    float lightProb;
-                    int li = selectLight(sc, rng.next(), &lightProb);
-                    float lu0 = rng.next(), lu1 = rng.next();
-                    V3 lp, lgn;
-                    Spec M;
-                    float areaPdf, edfVal, dist2;
-                    bool atInf = false;
-                    V3 shadowDir;
-                    if (li >= 0) {
-                        const DevPrim lpr = sc.prims[sc.lightPrims[li]];
-                        float su = sqrtf(lu0);
-                        float b0 = 1.0f - su, b1 = lu1 * su, b2 = 1.0f - b0 - b1;
-                        float4 p0 = sc.vpos[lpr.v0], p1 = sc.vpos[lpr.v1], p2 = sc.vpos[lpr.v2];
-                        lp = rn_bary(b0, V3{p0.x, p0.y, p0.z}, b1, V3{p1.x, p1.y, p1.z}, b2, V3{p2.x, p2.y, p2.z});
-                        float4 n0 = sc.vnrm[lpr.v0], n1 = sc.vnrm[lpr.v1], n2 = sc.vnrm[lpr.v2];
-                        V3 lz = normalize(b0 * V3{n0.x, n0.y, n0.z} + b1 * V3{n1.x, n1.y, n1.z} + b2 * V3{n2.x, n2.y, n2.z});
-                        lgn = V3{lpr.ngx, lpr.ngy, lpr.ngz};
-                        areaPdf = lpr.invArea;
-                        evalSpectrum(sc, sc.materials[lpr.material].emit, lambdas, M);
-                        V3 diff = lp - spN.p;
-                        dist2 = sqLength(diff);
-                        shadowDir = diff * (1.0f / sqrtf(dist2));
-                        edfVal = dot(lz, -shadowDir) > 0.0f ? kInvPiF : 0.0f;
-                    } else {
-                        float uvPdf, topPdf;
-                        uint32_t row, col;
-                        float d1 = sampleAlias(sc.envTopAlias, sc.envTopPDF, sc.envMapH, lu1, &topPdf, &row);
-                        float d0 = sampleAlias(sc.envRowAlias + (size_t)row * sc.envMapW,
-                                               sc.envRowPDF + (size_t)row * sc.envMapW, sc.envMapW, lu0, &uvPdf, &col);
-                        uvPdf *= topPdf;
-                        float phi = d0 * twoPi, theta = d1 * kPiF;
-                        float sph, cph, sth, cth;
-                        sincosf(phi, &sph, &cph);
-                        sincosf(theta, &sth, &cth);
-                        lp = V3{-sph * sth, cth, cph * sth};
-                        lgn = -lp;
-                        atInf = true;
-                        areaPdf = uvPdf / (2.0f * kPiF * kPiF * sth);
-                        envRadiance(sc, phi / twoPi, theta / kPiF, lambdas, M);
-                        edfVal = 1.0f;
-                        shadowDir = normalize(lp);
-                        dist2 = 1.0f;
-                    }
-                    float cosShading = absDot(shadowDir, spN.gn);
-                    float cosLight = absDot(shadowDir, lgn);
-                    if (cosShading * cosLight > 0) {
-                        float lightPdf = lightProb * areaPdf;
-                        V3 sdl = spN.frame.toLocal(shadowDir);
-                        Spec fs;
-                        bsdfEval<K>(B, q, sdl, fs);
-                        float bsdfPdfV = bsdfPdf<K>(B, q, sdl) * cosLight / dist2;
-                        float mis = 1.0f;
-                        if (!isinf(areaPdf))
-                            mis = (lightPdf * lightPdf) / (lightPdf * lightPdf + bsdfPdfV * bsdfPdfV);
-                        float G = cosShading * cosLight / dist2;
-                        float scale = G * mis / lightPdf;
-                        Spec c;
-                        bool nz = false;
-#pragma unroll
-                        for (int k = 0; k < kNumLambda; ++k) {
-                            c.v[k] = ((SLRGPU_ALPHA(k) * (M.v[k] * edfVal)) * fs.v[k]) * scale;
-                            nz |= c.v[k] != 0.0f;
-                        }
-                        if (nz) {
-                            storeSpec(ws.shContrib, p, c);
-                            float tmax;
-                            V3 sdir;
-                            if (atInf) {
-                                sdir = shadowDir;
-                                tmax = 3.402823466e+38f;
-                            } else {
-                                V3 dd = lp - spN.p;
-                                float dist = length(dd);
-                                sdir = dd * (1.0f / dist);
-                                tmax = dist * (1 - kRayEpsilon);
-                            }
-                            ws.shRay[2 * (size_t)p] = make_float4(spN.p.x, spN.p.y, spN.p.z, kRayEpsilon);
-                            ws.shRay[2 * (size_t)p + 1] = make_float4(sdir.x, sdir.y, sdir.z, tmax);
-                            shadow = true;
-                        }
-                    }
-                }
-                // BSDF sampling (PTRenderer.cpp:220-236).
-                float uc = rng.next(), u0 = rng.next(), u1 = rng.next();
-                BsdfSample bs;
-                Spec fs;
-                bsdfSample<K>(B, q, uc, u0, u1, &bs, fs);
-                if (bs.pdf == 0.0f || specIsZero(fs)) {
-                    alive = false;
-                } else {
-                    if ((bs.type & kDirDispersive) && !wlSelected) {
-                        bs.pdf /= kNumLambda;
-                        wlSelected = true;
-                    }
-                    float cg = absDot(bs.dir, q.gn);
-                    float r = 1.0f / bs.pdf;
-#pragma unroll
-                    for (int k = 0; k < kNumLambda; ++k) SLRGPU_ALPHA(k) *= (fs.v[k] * cg) * r;
-                    const SurfPoint spS = SLRGPU_SP();
-                    V3 nd = spS.frame.fromLocal(bs.dir);
-                    ws.ray[2 * (size_t)p] = make_float4(spS.p.x, spS.p.y, spS.p.z, kRayEpsilon);
-                    ws.ray[2 * (size_t)p + 1] = make_float4(nd.x, nd.y, nd.z, inf);
-                    ws.ps[p].prevPdf = bs.pdf;
-                    info = (uint32_t)sel | (wlSelected ? kInfoWlSelected : 0u) |
-                           (dirIsDelta(bs.type) ? kInfoPrevDelta : 0u) | (depth << kInfoDepthShift) | sceneBits;
-                    ws.ps[p].info = info;
-                    {
-                        Spec a2;
-#pragma unroll
-                        for (int k = 0; k < kNumLambda; ++k) a2.v[k] = SLRGPU_ALPHA(k);
-                        storeSpec(ws.alpha, p, a2);
-                    }
-                    extend = true;
-                }
-            }
-            ws.ps[p].rngCounter = rng.counter;
-        }
+        const uint32_t p = active ? inQueue[i] : 0;
+        if (active) shadeVertex<K, MULTI>(scArg, ws, p, maxDepth, scenes, sAlpha, sSurf, extend, shadow);
         queuePush(shQueue, shCount, p, active && shadow);
         queuePush(outQueue, outCount, p, active && extend);
+    }
+    if (!MULTI) waveEnd(beside);
+}
+
+// ---------------------------------------------------------------------------
+// The end of a wave: every remaining path to its last vertex in one launch.
+//
+// A bounce of few paths costs its kernels' latency, not their work: launching
+// persistent grids, cold instruction and node caches, and the slowest ray,
+// shaded vertex and shadow ray of the bounce one after another (on the
+// 176k-triangle terrain at 512 x 512 x 4 about 0.2 ms a bounce, whether it
+// holds ten paths or ten thousand).  So a bounce that starts with at most
+// SLRGPU_TAIL_PATHS paths is left to this kernel (the bounce kernels see the
+// same count and pass it by), where a thread takes a path through its
+// remaining vertices: closest hit, shading by class, shadow ray, with the
+// device functions of the bounce kernels.  The paths spread over as many
+// warps as there are: fewer lanes per warp diverge less and wait for fewer
+// others.  With more paths than lanes, a lane takes the next path of its
+// warp's range when its own ends.
+//
+// The counters of the bounces keep their meaning: every ray, class and shadow
+// ray is counted in the row of its bounce.
+//
+// Scenes with a smooth dielectric keep to the bounce kernels: compiled here,
+// its refracted direction differs in the last bit, and glass that stands on a
+// surface turns that into another path.  (The other kinds' paths are the
+// same: on the terrain of 176k triangles and the box no ray count changed with
+// every bounce below 131072 paths in this kernel.)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void countRows(uint32_t* counters, uint32_t row, uint32_t column, bool pred) {
+    // lanes of a warp are at the same bounce unless some took a new path
+    uint32_t rest = __ballot_sync(0xffffffffu, pred);
+    const uint32_t lane = threadIdx.x & 31;
+    while (rest) {
+        const int leader = __ffs(rest) - 1;
+        const uint32_t r = __shfl_sync(0xffffffffu, row, leader);
+        const uint32_t same = __ballot_sync(0xffffffffu, pred && row == r);
+        if ((int)lane == leader) atomicAdd(counters + (size_t)kCtrStride * r + column, (uint32_t)__popc(same));
+        rest &= ~same;
+    }
+}
+
+template <bool MULTI>
+__global__ void __launch_bounds__(256, 1) kTail(DevScene scArg, WaveState ws, uint32_t maxDepth,
+                                                                   const DevScene* __restrict__ scenes) {
+    __shared__ float sAlpha[SLRGPU_SHADE_SMEM_ALPHA ? kNumLambda * 256 : 1];
+    __shared__ float sSurf[SLRGPU_SHADE_SMEM_SP ? 15 * 256 : 1];
+    waveBegin(false);
+    if (ws.counters[kCtrTailRow] == 0) return;
+    const uint32_t b = ws.counters[kCtrTailRow] - 1;
+    const uint32_t n = ws.counters[(size_t)kCtrStride * b + kCtrExt];
+    const uint32_t* __restrict__ queue = ws.queue[b & 1];
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    // warps of different SMs first: consecutive ranges go to consecutive blocks
+    const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const uint32_t chunk = (n + warps - 1) / warps;
+    uint32_t next = min(warp * chunk, n);       // chunk x warps < n + warps fits 32 bits
+    const uint32_t end = min(next + chunk, n);
+    const uint32_t width = min(chunk, 32u);     // lanes that hold paths
+    uint32_t p = 0, row = b;
+    uint32_t rays = 0, shadows = 0;
+    bool live = false;
+    for (;;) {
+        // lanes without a path take the next of the warp's range
+        const bool want = !live && lane < width;
+        const uint32_t idle = __ballot_sync(0xffffffffu, want);
+        if (want) {
+            const uint32_t i = next + (uint32_t)__popc(idle & ((1u << lane) - 1));
+            if (i < end) {
+                p = queue[i];
+                row = b;
+                live = true;
+            }
+        }
+        next = min(next + (uint32_t)__popc(idle), end);
+        if (!__any_sync(0xffffffffu, live)) break;
+        int cls = -1;
+        if (live) {
+            const DevScene &sc = pathScene<MULTI>(scArg, scenes, MULTI ? ws.ps[p].info : 0u);
+            const float4 o = ws.ray[2 * (size_t)p], d = ws.ray[2 * (size_t)p + 1];
+            Hit h;
+            traceClosest(sc, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}, o.w, d.w, &h);
+            ++rays;
+            ws.hit[p] = make_float4(h.t, h.b1, h.b2, __uint_as_float(h.prim));
+            cls = hitClass(sc, ws, p, h.prim, maxDepth);
+        }
+        __syncwarp();
+        bool extend = false, shadow = false;
+#define SLRGPU_TAIL_CLASS(K)                                                                              \
+    if (__any_sync(0xffffffffu, cls == K)) {                                                              \
+        countRows(ws.counters, row, K, cls == K);                                                         \
+        if (cls == K) shadeVertex<K, MULTI>(scArg, ws, p, maxDepth, scenes, sAlpha, sSurf, extend, shadow); \
+        __syncwarp();                                                                                     \
+    }
+        SLRGPU_TAIL_CLASS(kMatMatte)
+        SLRGPU_TAIL_CLASS(kMatSpecularReflection)
+        SLRGPU_TAIL_CLASS(kMatGGXReflection)
+        SLRGPU_TAIL_CLASS(kMatGGXScattering)
+#undef SLRGPU_TAIL_CLASS
+        if (__any_sync(0xffffffffu, cls == kClassMiss)) {
+            countRows(ws.counters, row, kClassMiss, cls == kClassMiss);
+            if (cls == kClassMiss) shadeMiss<MULTI>(scArg, ws, p, scenes);
+            __syncwarp();
+        }
+        if (__any_sync(0xffffffffu, shadow)) {
+            countRows(ws.counters, row, kCtrShadow, shadow);
+            if (shadow) {
+                const DevScene &sc = pathScene<MULTI>(scArg, scenes, MULTI ? ws.ps[p].info : 0u);
+                const float4 o = ws.shRay[2 * (size_t)p], d = ws.shRay[2 * (size_t)p + 1];
+                ++shadows;
+                if (!traceAny(sc, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}, o.w, d.w)) {
+                    Spec c;
+                    loadSpec(ws.shContrib, p, c);
+                    addSpec(ws.L, p, c);
+                }
+            }
+            __syncwarp();
+        }
+        live = live && extend;
+        ++row;
+        countRows(ws.counters, row, kCtrExt, live);
+    }
+    rays = __reduce_add_sync(0xffffffffu, rays);
+    shadows = __reduce_add_sync(0xffffffffu, shadows);
+    if (lane == 0) {
+        if (rays) atomicAdd(&ws.stats[0], (unsigned long long)rays);
+        if (shadows) atomicAdd(&ws.stats[1], (unsigned long long)shadows);
     }
 }
 
 // ---------------------------------------------------------------------------
-#undef SLRGPU_ALPHA
-#undef SLRGPU_SP
 // Volumetric path tracing (VolumetricPTRenderer::Job::contribution,
 // libSLR/Renderer/VolumetricPTRenderer.cpp:146-296)
 // ---------------------------------------------------------------------------
@@ -832,6 +1028,7 @@ __global__ void __launch_bounds__(256, SLRGPU_VOLINTERACT_MIN_BLOCKS) kVolIntera
                                                                               const uint32_t* __restrict__ queue,
                                                                               const uint32_t* __restrict__ count,
                                                                               uint32_t* classCounts) {
+    waveBegin(false);
     const uint32_t n = *count;
     const float inf = __int_as_float(0x7f800000);
     const DevMedium &med = sc.medium;
@@ -885,9 +1082,10 @@ template <int K>
 __global__ void __launch_bounds__(256, SLRGPU_SHADEVOL_MIN_BLOCKS) kShadeVol(DevScene sc, WaveState ws, uint32_t maxDepth,
                                                  const uint32_t* __restrict__ inQueue,
                                                  const uint32_t* __restrict__ inCount, uint32_t* outQueue,
-                                                 uint32_t* outCount, uint32_t* shQueue, uint32_t* shCount) {
+                                                 uint32_t* outCount, uint32_t* shQueue, uint32_t* shCount,
+                                                 bool beside) {
+    waveBegin(beside);
     const uint32_t n = *inCount;
-    const uint32_t N = ws.N;
     const float inf = __int_as_float(0x7f800000);
     const float twoPi = 6.28318530717958647692f;
     const DevMedium &med = sc.medium;
@@ -1149,6 +1347,7 @@ __global__ void __launch_bounds__(256, SLRGPU_SHADEVOL_MIN_BLOCKS) kShadeVol(Dev
         queuePush(shQueue, shCount, p, active && shadow);
         queuePush(outQueue, outCount, p, active && extend);
     }
+    waveEnd(beside);
 }
 
 // Shadow rays of the volumetric integrator (Scene::testVisibility,
@@ -1159,9 +1358,11 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadowVol(DevSc
                                                                          const uint32_t* __restrict__ count,
                                                                          uint32_t* cursor, uint32_t* medQueue,
                                                                          uint32_t* medCount) {
+    waveBegin(true);
     const uint32_t n = *count;
 #if SLRGPU_TRACE_REFILL
-    if (sc.watertight) shadowRefill<false, true, true>(sc, ws, queue, n, cursor, nullptr, medQueue, medCount);
+    if (n == 0) {
+    } else if (sc.watertight) shadowRefill<false, true, true>(sc, ws, queue, n, cursor, nullptr, medQueue, medCount);
     else shadowRefill<false, false, true>(sc, ws, queue, n, cursor, nullptr, medQueue, medCount);
 #else
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
@@ -1185,6 +1386,7 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadowVol(DevSc
     }
 #endif
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ws.stats[1], (unsigned long long)n);
+    waveEnd(true);
 }
 
 // Medium transmittance of the unoccluded shadow rays: one ratio-tracking walk
@@ -1199,7 +1401,12 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadowVol(DevSc
 __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kShadowVolMedium(DevScene sc, WaveState ws,
                                                                                   const uint32_t* __restrict__ queue,
                                  const uint32_t* __restrict__ count, uint32_t* take, uint32_t bounce) {
+    waveBegin(true);
     const uint32_t n = *count * kNumLambda;
+    if (n == 0) {
+        waveEnd(true);
+        return;
+    }
     uint32_t poolNext = 0, poolEnd = 0;
     TrWalk q;
     uint32_t item = 0;
@@ -1241,6 +1448,7 @@ __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kShadowVolMediu
             }
         }
     }
+    waveEnd(true);
 }
 
 // Adds the wave's paths to the film: C = L * weight, dropped when not finite
@@ -1250,7 +1458,7 @@ __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kShadowVolMediu
 // Bound by the read of the paths' radiance and scalars (96 B a sample).  Four
 // lanes per pixel, each with four wavelengths and film bins: a sample's 64
 // bytes of radiance are one access of the quad, and a pixel's samples, which
-// lie next to each other, stream, four of them loaded ahead of the sums'
+// lie next to each other, stream, eight of them loaded ahead of the sums'
 // chain.  One thread per pixel took 0.42 ms on a 333 x 187 image with 24
 // samples, whose last pixel alone sums 576 (this kernel 0.23 ms), and sixteen
 // lanes repeated the per-sample work too often (1024 x 1024 x 64: 4.4 ms
@@ -1261,6 +1469,7 @@ constexpr uint32_t kFilmFirst = 1u;   // the film's sums start at zero: do not r
 constexpr uint32_t kFilmKeep = 2u;    // store sums and compensations for a later wave
 __global__ void __launch_bounds__(256) kAccumulate(WaveState ws, const __grid_constant__ WaveParams wpArg,
                                                    const WaveParams* __restrict__ wpDev, uint32_t flags, float* out) {
+    waveBegin(false);
     const WaveParams &wp = wpDev ? *wpDev : wpArg;
     const float recBinWidth = kNumLambda / (kWavelengthHigh - kWavelengthLow);
     constexpr uint32_t kLanes = 4, kBins = kNumLambda / kLanes;
@@ -1271,7 +1480,7 @@ __global__ void __launch_bounds__(256) kAccumulate(WaveState ws, const __grid_co
     for (uint32_t fp = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes; fp < wp.filmPixels; fp += step) {
         uint32_t k = 0;
         while (k + 1 < wp.numSegments && fp >= wp.seg[k + 1].filmBegin) ++k;
-        const WaveSegment &sg = wp.seg[k];
+        const WaveSegment sg = wp.seg[k];
         const uint32_t P = sg.width * sg.height;
         const uint32_t pix = fp - sg.filmBegin;
         float sum[kBins], comp[kBins];
@@ -1292,7 +1501,7 @@ __global__ void __launch_bounds__(256) kAccumulate(WaveState ws, const __grid_co
         const uint32_t yEnd = y + 1 == sg.height ? sg.gridH : y + 1;
         const uint32_t n = sg.samples * (xEnd - x) * (yEnd - y);
         uint32_t s = 0, gx = x, gy = y;
-        constexpr uint32_t kAhead = 4;
+        constexpr uint32_t kAhead = 8;
         for (uint32_t i0 = 0; i0 < n; i0 += kAhead) {
             float4 Lv[kAhead];
             float w[kAhead], off[kAhead];
@@ -1732,6 +1941,7 @@ fail:
 
 RenderEngine::~RenderEngine() {
     release();
+    bounceCounts.release();
     if (bpt) bptEngineDestroy(bpt);
 }
 
@@ -1750,6 +1960,49 @@ int RenderEngine::queueCounts(uint32_t* out, uint32_t capacity, uint32_t* rows) 
     CUDA_TRY(cudaMemcpy2D(out, kQueueCountColumns * sizeof(uint32_t), ws->counters, kCtrStride * sizeof(uint32_t),
                           kQueueCountColumns * sizeof(uint32_t), depthCapacity + 2, cudaMemcpyDeviceToHost));
     return SLRGPU_OK;
+}
+
+int BounceCounts::begin(uint32_t bounces) {
+    if (bounces > capacity) {
+        release();
+        const cudaError_t e = cudaMallocHost(&host, bounces * sizeof(*host));
+        if (e != cudaSuccess) {
+            host = nullptr;
+            setError(std::string("bounce counts: ") + cudaGetErrorString(e));
+            return SLRGPU_ERR_OUT_OF_MEMORY;
+        }
+        capacity = bounces;
+        std::memset(host, 0, bounces * sizeof(*host));
+        tag = 0;
+    }
+    ++tag;   // the waves of 2^32 before it are long complete
+    if (tag == 0) tag = 1;
+    return SLRGPU_OK;
+}
+
+cudaError_t BounceCounts::get(uint32_t bounce, cudaStream_t stream, uint32_t* count) {
+    const volatile unsigned long long* word = host + bounce;
+    for (uint32_t spins = 1;; ++spins) {
+        unsigned long long v = *word;
+        if ((uint32_t)(v >> 32) == tag) {
+            *count = (uint32_t)v;
+            return cudaSuccess;
+        }
+        if ((spins & 0xfff) == 0) {
+            // a stream that has run dry has written the word, or failed
+            const cudaError_t e = cudaStreamQuery(stream);
+            if (e == cudaErrorNotReady) continue;
+            v = *word;
+            *count = (uint32_t)v;
+            return e != cudaSuccess ? e : ((uint32_t)(v >> 32) == tag ? cudaSuccess : cudaErrorUnknown);
+        }
+    }
+}
+
+void BounceCounts::release() {
+    if (host) cudaFreeHost(host);
+    host = nullptr;
+    capacity = 0;
 }
 
 int RenderEngine::ensureFilm(uint32_t P) {
@@ -1797,6 +2050,7 @@ struct WaveGrids {
     int raygenM, shadowM, extendSortM, shadeMissM;
     int shadeSurfM[kNumShadeClasses - 1];
     int shadeVol[kNumClassQueues - 1];
+    int tail, tailM;
 };
 static const WaveGrids &waveGrids(int block) {
     static WaveGrids g;
@@ -1823,6 +2077,8 @@ static const WaveGrids &waveGrids(int block) {
         g.shadeSurf[kMatSpecularScattering] = gridFor((const void*)kShadeSurf<kMatSpecularScattering, false>, block);
         g.shadeSurf[kMatGGXReflection] = gridFor((const void*)kShadeSurf<kMatGGXReflection, false>, block);
         g.shadeSurf[kMatGGXScattering] = gridFor((const void*)kShadeSurf<kMatGGXScattering, false>, block);
+        g.tail = gridFor((const void*)kTail<false>, block);
+        g.tailM = gridFor((const void*)kTail<true>, block);
         g.raygenM = gridFor((const void*)kRaygen<true>, block);
         g.shadowM = gridFor((const void*)kShadow<true>, block);
         g.extendSortM = gridFor((const void*)kExtendSort<true>, block);
@@ -1912,25 +2168,66 @@ struct WaveSceneTable {
     bool env;
 };
 
+// Launches a kernel of a wave so that it may start before its predecessor has
+// completed; the kernel's own waits (waveBegin, waveEnd) order it.
+// Captured waves (the serving loop's) launch in plain order instead: their
+// slots' streams run side by side, and blocks that wait would hold the SMs
+// against the other slots' kernels (a burst of 24 requests: 43.6 ms plain,
+// 45.6 ms overlapped).
+struct WaveStream {
+    cudaStream_t stream;
+    bool overlap;
+};
+template <typename... P, typename... A>
+static void launchWaveKernel(void (*kernel)(P...), int grid, const WaveStream &ws, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = ws.stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = ws.overlap ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);   // errors: cudaGetLastError after the wave
+}
+
 // One bounce of the surface path tracer: closest hits sorted by shading
-// class, the shading kernels of the classes present, the shadow rays.
+// class, beside them the shadow rays of the bounce before (shadow rays end in
+// the radiance of their path, which the shading kernels are the next to
+// touch), then the shading kernels of the classes present beside each other.
+// The last bounce's vertices are past the maximum depth and cast no shadow
+// rays.
 template <bool MULTI>
 static void surfaceBounce(const DevScene &sc, const DevScene* scenes, uint32_t kindMask, bool env, const WaveState &w,
-                          uint32_t D, uint32_t* ctr, uint32_t* next, const uint32_t* inQueue, uint32_t* outQueue,
-                          cudaStream_t stream, LaunchMarks &lm, uint64_t &launches) {
-    const int block = 256;
-    const WaveGrids &g = waveGrids(block);
+                          uint32_t D, uint32_t b, uint32_t tailPaths, const WaveStream &stream, LaunchMarks &lm,
+                          uint64_t &launches) {
+    const WaveGrids &g = waveGrids(256);
+    uint32_t* ctr = w.counters + (size_t)kCtrStride * b;
+    uint32_t* next = ctr + kCtrStride;
+    const uint32_t* inQueue = w.queue[b & 1];
+    uint32_t* outQueue = w.queue[(b + 1) & 1];
     lm.begin(SLRGPU_KERNEL_EXTEND);
-    kExtendSort<MULTI><<<MULTI ? g.extendSortM : g.extendSort, block, 0, stream>>>(sc, w, inQueue, ctr + kCtrExt, ctr,
-                                                                                  ctr + kCtrExtTake, D, scenes);
+    launchWaveKernel(kExtendSort<MULTI>, MULTI ? g.extendSortM : g.extendSort, stream, sc, w, inQueue, ctr + kCtrExt,
+                     ctr, ctr + kCtrExtTake, D, tailPaths, scenes);
     lm.end();
     ++launches;
-    if (env) {
-        lm.begin(SLRGPU_KERNEL_SHADE);
-        kShadeMiss<MULTI><<<MULTI ? g.shadeMissM : g.shadeMiss, block, 0, stream>>>(
-            sc, w, w.classQueue + (size_t)kClassMiss * w.N, ctr + kClassMiss, scenes);
+    if (b > 0) {
+        uint32_t* last = ctr - kCtrStride;
+        lm.begin(SLRGPU_KERNEL_SHADOW);
+        launchWaveKernel(kShadow<MULTI>, MULTI ? g.shadowM : g.shadow, stream, sc, w, w.shadowQueue, last + kCtrShadow,
+                         last + kCtrShadowTake, scenes);
         lm.end();
         ++launches;
+    }
+    bool beside = false;
+    if (env) {
+        lm.begin(SLRGPU_KERNEL_SHADE);
+        launchWaveKernel(kShadeMiss<MULTI>, MULTI ? g.shadeMissM : g.shadeMiss, stream, sc, w,
+                         w.classQueue + (size_t)kClassMiss * w.N, ctr + kClassMiss, scenes, beside);
+        lm.end();
+        ++launches;
+        beside = true;
     }
     // One kernel per material kind present.
     for (int k = 0; k < kNumShadeClasses - 1; ++k) {
@@ -1938,9 +2235,9 @@ static void surfaceBounce(const DevScene &sc, const DevScene* scenes, uint32_t k
         const uint32_t* cq = w.classQueue + (size_t)k * w.N;
         const int grid = MULTI ? g.shadeSurfM[k] : g.shadeSurf[k];
         lm.begin(SLRGPU_KERNEL_SHADE);
-#define SLRGPU_SHADESURF(KK)                                                                                   \
-    kShadeSurf<KK, MULTI><<<grid, block, 0, stream>>>(sc, w, D, cq, ctr + k, outQueue, next + kCtrExt, w.shadowQueue, \
-                                                      ctr + kCtrShadow, scenes)
+#define SLRGPU_SHADESURF(KK)                                                                                  \
+    launchWaveKernel(kShadeSurf<KK, MULTI>, grid, stream, sc, w, D, cq, ctr + k, outQueue, next + kCtrExt, \
+                     w.shadowQueue, ctr + kCtrShadow, scenes, beside)
         switch (k) {
         case kMatMatte: SLRGPU_SHADESURF(kMatMatte); break;
         case kMatSpecularReflection: SLRGPU_SHADESURF(kMatSpecularReflection); break;
@@ -1951,97 +2248,146 @@ static void surfaceBounce(const DevScene &sc, const DevScene* scenes, uint32_t k
 #undef SLRGPU_SHADESURF
         lm.end();
         ++launches;
+        beside = true;
     }
-    lm.begin(SLRGPU_KERNEL_SHADOW);
-    kShadow<MULTI><<<MULTI ? g.shadowM : g.shadow, block, 0, stream>>>(sc, w, w.shadowQueue, ctr + kCtrShadow,
-                                                                       ctr + kCtrShadowTake, scenes);
-    lm.end();
-    ++launches;
 }
 
-static int runWave(const DeviceScene &ds0, const WaveState &w, const WaveParams &wp, uint32_t D, bool volumetric,
+// One bounce of the volumetric path tracer: closest hits, the medium collision
+// (or not), then the shading kernels of the vertex classes present; the shadow
+// rays of the bounce before (surface occlusion, then the transmittance of
+// the unoccluded ones, which wait in their own queue) run beside the closest
+// hits and the medium collisions.
+static void volumetricBounce(const DevScene &sc, uint32_t kindMask, const WaveState &w, uint32_t D, uint32_t b,
+                             const WaveStream &stream, LaunchMarks &lm, uint64_t &launches) {
+    const WaveGrids &g = waveGrids(256);
+    uint32_t* ctr = w.counters + (size_t)kCtrStride * b;
+    uint32_t* next = ctr + kCtrStride;
+    uint32_t* last = b > 0 ? ctr - kCtrStride : nullptr;
+    const uint32_t* inQueue = w.queue[b & 1];
+    uint32_t* outQueue = w.queue[(b + 1) & 1];
+    uint32_t* medQueue = w.classQueue + (size_t)kQueueMedShadow * w.N;
+    lm.begin(SLRGPU_KERNEL_EXTEND);
+    launchWaveKernel(kExtend, g.extend, stream, sc, w, inQueue, ctr + kCtrExt, ctr + kCtrExtTake);
+    lm.end();
+    ++launches;
+    if (last) {
+        lm.begin(SLRGPU_KERNEL_SHADOW);
+        launchWaveKernel(kShadowVol, g.shadowVol, stream, sc, w, w.shadowQueue, last + kCtrShadow,
+                         last + kCtrShadowTake, medQueue, last + kCtrMedShadow);
+        lm.end();
+        ++launches;
+    }
+    lm.begin(SLRGPU_KERNEL_SHADE);
+    launchWaveKernel(kVolInteract, g.volInteract, stream, sc, w, inQueue, ctr + kCtrExt, ctr);
+    lm.end();
+    ++launches;
+    if (last) {
+        lm.begin(SLRGPU_KERNEL_SHADOW);
+        launchWaveKernel(kShadowVolMedium, g.shadowVolMedium, stream, sc, w, medQueue, last + kCtrMedShadow,
+                         last + kCtrMedTake, b - 1);
+        lm.end();
+        ++launches;
+    }
+    bool beside = false;
+    for (int k = 0; k < kNumClassQueues - 1; ++k) {
+        const bool present = k < kClassMiss ? (kindMask & (1u << k)) != 0
+                                            : (k == kClassMiss ? sc.envPresent != 0 : sc.medium.present != 0);
+        if (!present) continue;
+        const uint32_t* cq = w.classQueue + (size_t)k * w.N;
+        lm.begin(SLRGPU_KERNEL_SHADE);
+#define SLRGPU_SHADEVOL(KK)                                                                                      \
+    launchWaveKernel(kShadeVol<KK>, g.shadeVol[KK], stream, sc, w, D, cq, ctr + k, outQueue, next + kCtrExt, \
+                     w.shadowQueue, ctr + kCtrShadow, beside)
+        switch (k) {
+        case 0: SLRGPU_SHADEVOL(0); break;
+        case 1: SLRGPU_SHADEVOL(1); break;
+        case 2: SLRGPU_SHADEVOL(2); break;
+        case 3: SLRGPU_SHADEVOL(3); break;
+        case 4: SLRGPU_SHADEVOL(4); break;
+        case 5: SLRGPU_SHADEVOL(5); break;
+        default: SLRGPU_SHADEVOL(6); break;
+        }
+#undef SLRGPU_SHADEVOL
+        lm.end();
+        ++launches;
+        beside = true;
+    }
+}
+
+// Bounces of the surface path tracer that start with at most this many
+// paths go to kTail.  A 64 x 64 x 1 frame of the box (4096 paths): 392 us with
+// bounce kernels alone, 237 us in the tail kernel; the 176k-triangle terrain
+// at 512 x 512 x 4: 2458 us with bounce kernels alone, 2397 us at this line,
+// 2935 us with the line at 10000, where the tail's mixed warps cost more than
+// the bounces' launches.
+#ifndef SLRGPU_TAIL_PATHS
+#define SLRGPU_TAIL_PATHS 4096u
+#endif
+
+static int runWave(const DeviceScene &ds0, const WaveState &w0, const WaveParams &wp, uint32_t D, bool volumetric,
                    bool watertight, cudaStream_t stream, LaunchMarks &lm, uint64_t* launchCount,
                    const WaveParams* wpDev = nullptr, const float* rngTape = nullptr,
-                   const WaveSceneTable* multi = nullptr, uint32_t filmFlags = kFilmKeep, float* filmOut = nullptr) {
+                   const WaveSceneTable* multi = nullptr, uint32_t filmFlags = kFilmKeep, float* filmOut = nullptr,
+                   BounceCounts* counts = nullptr) {
     // the scene as the kernels see it, with the triangle test chosen
     struct { DevScene sc; uint32_t kindMask; } ds{ds0.sc, ds0.kindMask};
     ds.sc.watertight = watertight ? 1u : 0u;
     ds.sc.rngTape = rngTape;
-    const int block = 256;
-    const WaveGrids &g = waveGrids(block);
+    const WaveGrids &g = waveGrids(256);
+    const uint32_t kinds = multi ? multi->kindMask : ds.kindMask;
+    const uint32_t tailPaths = volumetric || (kinds >> kMatSpecularScattering & 1u) ? 0u : SLRGPU_TAIL_PATHS;
+    const WaveStream order{stream, wpDev == nullptr && multi == nullptr};
     uint64_t launches = 0;
-    CUDA_TRY(cudaMemsetAsync(w.counters, 0, (size_t)kCtrStride * (D + 2) * sizeof(uint32_t), stream));
+    CUDA_TRY(cudaMemsetAsync(w0.counters, 0, (size_t)kCtrStride * (D + 2) * sizeof(uint32_t), stream));
     if (multi && volumetric) {
         setError("waves of several scenes are for the surface path tracer");
         return SLRGPU_ERR_INVALID_ARGUMENT;
     }
+    WaveState w = w0;
+    w.hostCounts = nullptr;
+    if (counts) {
+        if (int rc = counts->begin(D + 1)) return rc;
+        w.hostCounts = counts->host;
+        w.hostTag = counts->tag;
+    }
     lm.begin(SLRGPU_KERNEL_RAYGEN);
     if (multi)
-        kRaygen<true><<<g.raygenM, block, 0, stream>>>(ds.sc, w, wp, wpDev, multi->dev, volumetric);
+        kRaygen<true><<<g.raygenM, 256, 0, stream>>>(ds.sc, w, wp, wpDev, multi->dev, volumetric, tailPaths);
     else
-        kRaygen<false><<<g.raygen, block, 0, stream>>>(ds.sc, w, wp, wpDev, nullptr, volumetric);
+        kRaygen<false><<<g.raygen, 256, 0, stream>>>(ds.sc, w, wp, wpDev, nullptr, volumetric, tailPaths);
     lm.end();
     ++launches;
-    for (uint32_t b = 0; b <= D; ++b) {
-        TraceRange range("bounce %u", b);
-        uint32_t* ctr = w.counters + (size_t)kCtrStride * b;
-        uint32_t* next = ctr + kCtrStride;
-        uint32_t* inQueue = w.queue[b & 1];
-        uint32_t* outQueue = w.queue[(b + 1) & 1];
-        if (volumetric) {
-            lm.begin(SLRGPU_KERNEL_EXTEND);
-            kExtend<<<g.extend, block, 0, stream>>>(ds.sc, w, inQueue, ctr + kCtrExt, ctr + kCtrExtTake);
-            lm.end();
-            // the medium collision (or not), then one shading kernel per
-            // vertex class present
-            lm.begin(SLRGPU_KERNEL_SHADE);
-            kVolInteract<<<g.volInteract, block, 0, stream>>>(ds.sc, w, inQueue, ctr + kCtrExt, ctr);
-            lm.end();
-            launches += 2;
-            for (int k = 0; k < kNumClassQueues - 1; ++k) {
-                const bool present = k < kClassMiss ? (ds.kindMask & (1u << k)) != 0
-                                                    : (k == kClassMiss ? ds.sc.envPresent != 0 : ds.sc.medium.present != 0);
-                if (!present) continue;
-                const uint32_t* cq = w.classQueue + (size_t)k * w.N;
-                lm.begin(SLRGPU_KERNEL_SHADE);
-#define SLRGPU_SHADEVOL(KK)                                                                              \
-    kShadeVol<KK><<<g.shadeVol[KK], block, 0, stream>>>(ds.sc, w, D, cq, ctr + k, outQueue, next + kCtrExt, \
-                                                        w.shadowQueue, ctr + kCtrShadow)
-                switch (k) {
-                case 0: SLRGPU_SHADEVOL(0); break;
-                case 1: SLRGPU_SHADEVOL(1); break;
-                case 2: SLRGPU_SHADEVOL(2); break;
-                case 3: SLRGPU_SHADEVOL(3); break;
-                case 4: SLRGPU_SHADEVOL(4); break;
-                case 5: SLRGPU_SHADEVOL(5); break;
-                default: SLRGPU_SHADEVOL(6); break;
-                }
-#undef SLRGPU_SHADEVOL
-                lm.end();
-                ++launches;
-            }
-            // unoccluded shadow rays that cross the medium wait in their own queue
-            uint32_t* medQueue = w.classQueue + (size_t)kQueueMedShadow * w.N;
-            lm.begin(SLRGPU_KERNEL_SHADOW);
-            kShadowVol<<<g.shadowVol, block, 0, stream>>>(ds.sc, w, w.shadowQueue, ctr + kCtrShadow,
-                                                          ctr + kCtrShadowTake, medQueue, ctr + kCtrMedShadow);
-            lm.end();
-            lm.begin(SLRGPU_KERNEL_SHADOW);
-            kShadowVolMedium<<<g.shadowVolMedium, block, 0, stream>>>(ds.sc, w, medQueue, ctr + kCtrMedShadow,
-                                                                      ctr + kCtrMedTake, b);
-            lm.end();
-            launches += 2;
-            continue;
+    // A wave that starts with few paths has no bounce kernels at all; another
+    // one launches them until it sees (one bounce late, so that the GPU never
+    // waits for the host) that a bounce has no paths or was left to the tail
+    // kernel, or, where the host may not look (graph capture, the
+    // asynchronous entry point), for every bounce.
+    const bool tailOnly = !volumetric && wpDev == nullptr && wp.numPaths <= tailPaths;
+    for (uint32_t b = 0; b <= D && !tailOnly; ++b) {
+        if (counts && b >= 2) {
+            uint32_t left = 0;
+            CUDA_TRY(counts->get(b - 1, stream, &left));
+            if (left <= tailPaths) break;
         }
-        if (multi)
-            surfaceBounce<true>(ds.sc, multi->dev, multi->kindMask, multi->env, w, D, ctr, next, inQueue, outQueue,
-                                stream, lm, launches);
+        TraceRange range("bounce %u", b);
+        if (volumetric)
+            volumetricBounce(ds.sc, ds.kindMask, w, D, b, order, lm, launches);
+        else if (multi)
+            surfaceBounce<true>(ds.sc, multi->dev, multi->kindMask, multi->env, w, D, b, tailPaths, order, lm,
+                                launches);
         else
-            surfaceBounce<false>(ds.sc, nullptr, ds.kindMask, ds.sc.envPresent != 0, w, D, ctr, next, inQueue,
-                                 outQueue, stream, lm, launches);
+            surfaceBounce<false>(ds.sc, nullptr, ds.kindMask, ds.sc.envPresent != 0, w, D, b, tailPaths, order, lm,
+                                 launches);
+    }
+    if (tailPaths > 0) {
+        lm.begin(SLRGPU_KERNEL_SHADE);
+        if (multi) launchWaveKernel(kTail<true>, g.tailM, order, ds.sc, w, D, multi->dev);
+        else launchWaveKernel(kTail<false>, g.tail, order, ds.sc, w, D, (const DevScene*)nullptr);
+        lm.end();
+        ++launches;
     }
     lm.begin(SLRGPU_KERNEL_ACCUMULATE);
-    kAccumulate<<<g.accumulate, block, 0, stream>>>(w, wp, wpDev, filmFlags, filmOut);
+    launchWaveKernel(kAccumulate, g.accumulate, order, w, wp, wpDev, filmFlags, filmOut);
     lm.end();
     ++launches;
     *launchCount += launches;
@@ -2056,7 +2402,8 @@ static int runWave(const DeviceScene &ds0, const WaveState &w, const WaveParams 
 // stored where a later wave or, with `keepLast`, the caller reads them.
 static int runWaves(const DeviceScene &ds, const slrgpu_settings &s, const WavePlan &pl, const WaveState &w,
                     float* filmSum, float* filmComp, float* film, bool resume, bool keepLast, cudaStream_t stream,
-                    LaunchMarks &lm, uint64_t* launches, const float* rngTape = nullptr) {
+                    LaunchMarks &lm, uint64_t* launches, const float* rngTape = nullptr,
+                    BounceCounts* counts = nullptr) {
     for (uint32_t base = 0; base < s.spp; base += pl.S) {
         TraceRange range("wave: samples %u..%u", s.sample_base + base, s.sample_base + std::min(s.spp, base + pl.S));
         WaveParams wp;
@@ -2081,7 +2428,7 @@ static int runWaves(const DeviceScene &ds, const slrgpu_settings &s, const WaveP
         const bool last = s.spp - base <= pl.S;
         const uint32_t filmFlags = (base == 0 && !resume ? kFilmFirst : 0u) | (!last || keepLast ? kFilmKeep : 0u);
         int rc = runWave(ds, w, wp, s.max_depth, s.volumetric != 0, (s.flags & SLRGPU_FLAG_WATERTIGHT) != 0,
-                         stream, lm, launches, nullptr, rngTape, nullptr, filmFlags, last ? film : nullptr);
+                         stream, lm, launches, nullptr, rngTape, nullptr, filmFlags, last ? film : nullptr, counts);
         if (rc != SLRGPU_OK) return rc;
     }
     return SLRGPU_OK;
@@ -2159,7 +2506,7 @@ int RenderEngine::render(const DeviceScene &ds, const slrgpu_settings &s, float*
         ++launches;
     } else {
         rc = runWaves(ds, s, pl, *ws, filmSum, filmComp, dst, filmState != nullptr, filmState != nullptr, stream, lm,
-                      &launches, rngTape);
+                      &launches, rngTape, &bounceCounts);
         if (rc != SLRGPU_OK) return rc;
     }
     CUDA_TRY(cudaGetLastError());
