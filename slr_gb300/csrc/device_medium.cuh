@@ -88,62 +88,53 @@ __device__ __forceinline__ bool mediumIntersectBoundary(const DevMedium &m, V3 o
 }
 
 // ---- super-voxel traversal -------------------------------------------------
+// The walk is bound by its instructions: with 13 of 32 lanes doing useful work
+// per instruction (lanes are in different cells, collisions and
+// iterations), every instruction of a cell counts.  So its state is scalars that
+// stay in registers (arrays indexed by the crossed axis lived in local
+// memory), it is inlined, where the medium's constants are operands from the
+// constant bank, and a cell's corner differences come ready made in three
+// loads instead of nine loads and fourteen additions.  @@MEDFIG@@
 struct SvWalk {
-    int sv[3];
-    float maxt[3];
+    int x, y, z;            // the cell
+    float tx, ty, tz;       // distances to its exit planes
 };
 
 struct SvSetup {
-    int step[3];
-    int outside[3];
-    float invD[3];      // 1 / direction: the plane distances are multiplications
+    V3 invD;                // 1 / direction: the plane distances are multiplications
     SvWalk init;
 };
+
+__device__ __forceinline__ float svPlane(float bmin, float width, int cell, bool up) {
+    return bmin + width * (cell + (up ? 1 : 0));
+}
 
 __device__ __forceinline__ void svSetup(const DevMedium &m, V3 org, V3 dir, float dmin, SvSetup &s) {
     V3 p = mediumLocal(m, org + dmin * dir);
     p = V3{fminf(fmaxf(p.x, 0.0f), 1.0f), fminf(fmaxf(p.y, 0.0f), 1.0f), fminf(fmaxf(p.z, 0.0f), 1.0f)};
-    const uint32_t n[3] = {m.svx, m.svy, m.svz};
-    const float lp[3] = {p.x, p.y, p.z}, o[3] = {org.x, org.y, org.z}, d[3] = {dir.x, dir.y, dir.z};
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        s.init.sv[i] = min((int)(lp[i] * (n[i] - 1)), (int)n[i] - 2);
-        s.invD[i] = 1.0f / d[i];
-        if (d[i] > 0) {
-            s.step[i] = 1;
-            s.outside[i] = (int)n[i] - 1;
-            float plane = m.bmin[i] + m.svWidth[i] * (s.init.sv[i] + 1);
-            s.init.maxt[i] = (plane - o[i]) * s.invD[i];
-        } else {
-            s.step[i] = -1;
-            s.outside[i] = -1;
-            float plane = m.bmin[i] + m.svWidth[i] * (s.init.sv[i] + 0);
-            s.init.maxt[i] = (plane - o[i]) * s.invD[i];
-        }
-    }
+    s.invD = V3{1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z};
+    s.init.x = min((int)(p.x * (m.svx - 1)), (int)m.svx - 2);
+    s.init.y = min((int)(p.y * (m.svy - 1)), (int)m.svy - 2);
+    s.init.z = min((int)(p.z * (m.svz - 1)), (int)m.svz - 2);
+    s.init.tx = (svPlane(m.bmin[0], m.svWidth[0], s.init.x, dir.x > 0) - org.x) * s.invD.x;
+    s.init.ty = (svPlane(m.bmin[1], m.svWidth[1], s.init.y, dir.y > 0) - org.y) * s.invD.y;
+    s.init.tz = (svPlane(m.bmin[2], m.svWidth[2], s.init.z, dir.z > 0) - org.z) * s.invD.z;
 }
 
 // Cubic in the segment parameter of the trilinear super-voxel majorant
 // between entry and exit (plus the cell's maximum difference).
-__device__ __forceinline__ void svPolyCoeffs(const DevMedium &m, V3 entry, V3 exit, const int cell[3], float c[4]) {
-    const uint32_t sx = m.svx, sxy = m.svx * m.svy;
-    const float* s = m.superVoxels;
-    const int i0 = sxy * cell[2] + sx * cell[1] + cell[0];
-    float d000 = __ldg(s + i0), d100 = __ldg(s + i0 + 1), d010 = __ldg(s + i0 + sx), d110 = __ldg(s + i0 + sx + 1);
-    float d001 = __ldg(s + i0 + sxy), d101 = __ldg(s + i0 + sxy + 1), d011 = __ldg(s + i0 + sxy + sx),
-          d111 = __ldg(s + i0 + sxy + sx + 1);
-    V3 base = V3{m.bmin[0] + cell[0] * m.svWidth[0], m.bmin[1] + cell[1] * m.svWidth[1],
-                 m.bmin[2] + cell[2] * m.svWidth[2]};
+__device__ __forceinline__ void svPolyCoeffs(const DevMedium &m, V3 entry, V3 exit, const SvWalk &w, float c[4]) {
+    const float4* cp = reinterpret_cast<const float4*>(
+        m.cells + ((m.svx - 1) * (m.svy - 1) * w.z + (m.svx - 1) * w.y + w.x));
+    const float4 q0 = __ldg(cp), q1 = __ldg(cp + 1);
+    const float maxDiff = __ldg(reinterpret_cast<const float*>(cp + 2));
+    const float dxyz = q0.x, dxy = q0.y, dxz = q0.z, dyz = q0.w, dx = q1.x, dy = q1.y, dz = q1.z, d000 = q1.w;
+    V3 base = V3{m.bmin[0] + w.x * m.svWidth[0], m.bmin[1] + w.y * m.svWidth[1], m.bmin[2] + w.z * m.svWidth[2]};
     V3 ep = V3{(entry.x - base.x) * m.invSvWidth[0], (entry.y - base.y) * m.invSvWidth[1],
                (entry.z - base.z) * m.invSvWidth[2]};
     V3 op = V3{(exit.x - base.x) * m.invSvWidth[0], (exit.y - base.y) * m.invSvWidth[1],
                (exit.z - base.z) * m.invSvWidth[2]};
     V3 dl = op - ep;
-    float dxyz = d111 - d011 - d101 - d110 + d001 + d010 + d100 - d000;
-    float dxy = d000 - d100 - d010 + d110;
-    float dxz = d000 - d100 - d001 + d101;
-    float dyz = d000 - d010 - d001 + d011;
-    float dx = d100 - d000, dy = d010 - d000, dz = d001 - d000;
     c[3] = dxyz * dl.x * dl.y * dl.z;
     c[2] = ((ep.z * dl.x * dl.y + ep.y * dl.x * dl.z + ep.x * dl.y * dl.z) * dxyz + dxy * dl.x * dl.y +
             dxz * dl.x * dl.z + dyz * dl.y * dl.z);
@@ -152,7 +143,7 @@ __device__ __forceinline__ void svPolyCoeffs(const DevMedium &m, V3 entry, V3 ex
             (ep.z * dl.y + ep.y * dl.z) * dyz);
     c[0] = (ep.x * ep.y * ep.z * dxyz + ep.x * ep.y * dxy + ep.x * ep.z * dxz + ep.y * ep.z * dyz + ep.x * dx +
             ep.y * dy + ep.z * dz + d000);
-    c[0] += __ldg(m.maxDiff + (m.svx - 1) * (m.svy - 1) * cell[2] + (m.svx - 1) * cell[1] + cell[0]);
+    c[0] += maxDiff;
 }
 
 // traverseSuperVoxels (DensityGridMediumDistribution.cpp:208-367): samples a
@@ -160,8 +151,8 @@ __device__ __forceinline__ void svPolyCoeffs(const DevMedium &m, V3 entry, V3 ex
 // false (and *dist = dmax) when the walk leaves the segment.
 constexpr int kMaxSvSteps = 4096;
 
-static __device__ __noinline__ bool svTraverse(const DevMedium &m, V3 org, V3 dir, float dmin, float dmax, float u,
-                                        float sigma, const SvSetup &s, SvWalk &w, float* dist, float* majorant) {
+__device__ __forceinline__ bool svTraverse(const DevMedium &m, V3 org, V3 dir, float dmin, float dmax, float u,
+                                           float sigma, const SvSetup &s, SvWalk &w, float* dist, float* majorant) {
     float sampledOD = -logf(1 - u);
     if (sampledOD == 0.0f) {
         V3 q = org + (*dist) * dir;
@@ -177,24 +168,36 @@ static __device__ __noinline__ bool svTraverse(const DevMedium &m, V3 org, V3 di
         entryP = exitP;
         entryDist = exitDist;
         entryOD = exitOD;
-        const uint32_t cond = (uint32_t)(w.maxt[0] < w.maxt[1]) | ((uint32_t)(w.maxt[0] < w.maxt[2]) << 1) |
-                              ((uint32_t)(w.maxt[1] < w.maxt[2]) << 2);
-        // axisMap[cond] = {2, 2, 2, 0, 1, 2, 1, 0}, one nibble per entry
-        const int axis = (0x01210222u >> (4 * cond)) & 0xf;
-        exitDist = w.maxt[axis];
+        // The axis whose plane comes first; of equal distances the later
+        // axis, as the reference's comparison table has it.
+        const bool isX = w.tx < w.ty && w.tx < w.tz;
+        const bool isY = !(w.tx < w.ty) && w.ty < w.tz;
+        exitDist = isX ? w.tx : (isY ? w.ty : w.tz);
         exitP = org + exitDist * dir;
-        svPolyCoeffs(m, entryP, exitP, w.sv, c);
+        svPolyCoeffs(m, entryP, exitP, w, c);
         exitOD += (exitDist - entryDist) * sigma * (c[0] + c[1] * 0.5f + c[2] * kThird + c[3] * 0.25f);
         if (exitOD >= sampledOD) break;
-        w.sv[axis] += s.step[axis];
-        if (w.sv[axis] == s.outside[axis] || exitDist >= dmax || ++steps > kMaxSvSteps) {
+        // one cell along the axis; out of the grid on either side ends the walk
+        const float da = isX ? dir.x : (isY ? dir.y : dir.z);
+        const bool up = da > 0;
+        const int cell = (isX ? w.x : (isY ? w.y : w.z)) + (up ? 1 : -1);
+        const int outside = up ? (int)(isX ? m.svx : (isY ? m.svy : m.svz)) - 1 : -1;
+        if (cell == outside || exitDist >= dmax || ++steps > kMaxSvSteps) {
+            if (isX) w.x = cell;
+            else if (isY) w.y = cell;
+            else w.z = cell;
             *dist = dmax;
             *majorant = __int_as_float(0x7fc00000);
             return false;
         }
-        float plane = m.bmin[axis] + m.svWidth[axis] * (w.sv[axis] + (s.step[axis] == 1 ? 1 : 0));
-        const float oa = axis == 0 ? org.x : (axis == 1 ? org.y : org.z);
-        w.maxt[axis] = (plane - oa) * s.invD[axis];
+        const float bmin = isX ? m.bmin[0] : (isY ? m.bmin[1] : m.bmin[2]);
+        const float width = isX ? m.svWidth[0] : (isY ? m.svWidth[1] : m.svWidth[2]);
+        const float oa = isX ? org.x : (isY ? org.y : org.z);
+        const float inv = isX ? s.invD.x : (isY ? s.invD.y : s.invD.z);
+        const float t = (svPlane(bmin, width, cell, up) - oa) * inv;
+        if (isX) { w.x = cell; w.tx = t; }
+        else if (isY) { w.y = cell; w.ty = t; }
+        else { w.z = cell; w.tz = t; }
     }
     // Regula falsi on the integrated majorant.
     float pLow = 0.0f, pHigh = 1.0f, odLow = entryOD, odHigh = exitOD;
@@ -260,25 +263,24 @@ __device__ __noinline__ bool mediumInteractSegment(const DevMedium &m, V3 org, V
         const float hitDist = fminf(sd, dmax);
         sd = dmin;
         w = s.init;
-        Spec mc = specConst(1.0f);
         // The walk state is shared across the wavelengths, so only the first
         // wavelength other than the selected one takes steps (the reference's
         // loop at DensityGridMediumDistribution.cpp:487-510 never resets it).
-        for (int wl = 0; wl < kNumLambda; ++wl) {
-            if (wl == sel) continue;
-            const float sigWl = specAt(sigmaE, wl);
-            while (sd < hitDist) {
-                float maj;
-                bool tent = svTraverse(m, org, dir, sd, hitDist, rng.next(), sigWl, s, w, &sd, &maj);
-                if (tent) {
-                    V3 q = org + sd * dir;
-                    float dens = mediumDensity(m, mediumLocal(m, q));
-                    float prob = (sigWl * dens - sigSel * dens) / maj;
-                    if (maj != 0.0f) mc.v[wl] *= (1.0f - prob);
-                }
+        const int wl = sel == 0 ? 1 : 0;
+        const float sigWl = wl == 0 ? sigmaE.v[0] : sigmaE.v[1];
+        float mc = 1.0f;
+        while (sd < hitDist) {
+            float maj;
+            bool tent = svTraverse(m, org, dir, sd, hitDist, rng.next(), sigWl, s, w, &sd, &maj);
+            if (tent) {
+                V3 q = org + sd * dir;
+                float dens = mediumDensity(m, mediumLocal(m, q));
+                float prob = (sigWl * dens - sigSel * dens) / maj;
+                if (maj != 0.0f) mc *= (1.0f - prob);
             }
         }
-        thr = mc;
+#pragma unroll
+        for (int k = 0; k < kNumLambda; ++k) thr.v[k] = k == wl ? mc : 1.0f;
     }
     if (hit) {
         float r = 1.0f / extAt;

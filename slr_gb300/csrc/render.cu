@@ -1871,6 +1871,7 @@ int uploadScene(const HostScene &hs, const BuiltScene &bs, DeviceScene* ds) {
         UP(hs.medium.density, medium.density);
         UP(bs.superVoxels.corners, medium.superVoxels);
         UP(bs.superVoxels.maxDiff, medium.maxDiff);
+        UP(bs.superVoxels.cells, medium.cells);
         m.present = 1;
         m.nx = hs.medium.nx; m.ny = hs.medium.ny; m.nz = hs.medium.nz;
         m.svx = bs.superVoxels.svx; m.svy = bs.superVoxels.svy; m.svz = bs.superVoxels.svz;

@@ -1236,6 +1236,29 @@ void buildSuperVoxels(const HostMedium &m, HostSuperVoxels* sv) {
         }
     }
     sv->maxDiff = diffs;
+    // The corner differences of every cell: sums alone, each rounded here as
+    // the walk would round it.
+    sv->cells.resize(ncell);
+    for (uint32_t cz = 0; cz < svz - 1; ++cz)
+        for (uint32_t cy = 0; cy < svy - 1; ++cy)
+            for (uint32_t cx = 0; cx < svx - 1; ++cx) {
+                const size_t cell = ((size_t)cz * (svy - 1) + cy) * (svx - 1) + cx;
+                const float* c = sv->corners.data() + ((size_t)cz * svy + cy) * svx + cx;
+                const size_t sy = svx, sz = (size_t)svx * svy;
+                const float d000 = c[0], d100 = c[1], d010 = c[sy], d110 = c[sy + 1];
+                const float d001 = c[sz], d101 = c[sz + 1], d011 = c[sz + sy], d111 = c[sz + sy + 1];
+                SvCell &o = sv->cells[cell];
+                o.dxyz = d111 - d011 - d101 - d110 + d001 + d010 + d100 - d000;
+                o.dxy = d000 - d100 - d010 + d110;
+                o.dxz = d000 - d100 - d001 + d101;
+                o.dyz = d000 - d010 - d001 + d011;
+                o.dx = d100 - d000;
+                o.dy = d010 - d000;
+                o.dz = d001 - d000;
+                o.d000 = d000;
+                o.maxDiff = diffs[cell];
+                o.pad0 = o.pad1 = o.pad2 = 0.0f;
+            }
 }
 
 // ============================================================================

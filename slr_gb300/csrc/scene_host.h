@@ -111,6 +111,7 @@ struct HostSuperVoxels {
     float width[3];
     std::vector<float> corners;    // [svz][svy][svx]
     std::vector<float> maxDiff;    // [svz-1][svy-1][svx-1]
+    std::vector<SvCell> cells;     // the same cells as the device's walks read them
 };
 void buildSuperVoxels(const HostMedium &m, HostSuperVoxels* sv);
 // Trilinear density at a normalised position in [0,1]^3 (0 outside).

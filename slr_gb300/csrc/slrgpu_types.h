@@ -114,6 +114,15 @@ struct EnvTexel {
     float s, t, scale;
 };
 
+// One super-voxel cell (48 B, three 128-bit loads): the corner differences that
+// its trilinear majorant's cubic along a ray is built from, and the cell's
+// maximum difference.
+struct SvCell {
+    float dxyz, dxy, dxz, dyz;
+    float dx, dy, dz, d000;
+    float maxDiff, pad0, pad1, pad2;
+};
+
 // Heterogeneous medium: density grid over an axis-aligned box with a
 // super-voxel majorant grid (DensityGridMediumDistribution).
 struct DevMedium {
@@ -127,6 +136,7 @@ struct DevMedium {
     const float* density;         // [nz][ny][nx]
     const float* superVoxels;     // [svz][svy][svx]
     const float* maxDiff;         // [svz-1][svy-1][svx-1]
+    const SvCell* cells;          // [svz-1][svy-1][svx-1]
     int32_t sigmaS, sigmaE;       // spectrum ids
     float g;                      // Henyey-Greenstein asymmetry
     float importance;             // emitting media weight (0: none emit)
