@@ -1061,43 +1061,31 @@ __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kVbptMedium(Dev
                                                                            const uint32_t* __restrict__ medCount,
                                                                            uint32_t* take) {
     const uint32_t n = *medCount * kNumLambda;
-    uint32_t poolNext = 0, poolEnd = 0;
-    TrWalk q;
-    uint32_t slot = 0;
-    int wl = 0;
-    float cw = 0.0f;
-    bool walking = false, exhausted = false;
-    for (;;) {
-        for (;;) {
-            const bool need = !walking && !exhausted;
-            if (!__any_sync(0xffffffffu, need)) break;
-            const uint32_t item = trTake(need, take, poolNext, poolEnd);
-            if (!need) continue;
-            if (item >= n) {
-                exhausted = true;
-                continue;
-            }
-            slot = st.mQueue[item / kNumLambda];
-            wl = (int)(item % kNumLambda);
-            cw = reinterpret_cast<const float*>(st.cContrib)[(size_t)slot * kNumLambda + wl];
-            if (cw == 0.0f) continue;
+    trRun(
+        sc.medium, n, take,
+        [&](uint32_t item, TrWalk &q) {
+            const uint32_t slot = st.mQueue[item / kNumLambda];
+            const int wl = (int)(item % kNumLambda);
+            const float cw = reinterpret_cast<const float*>(st.cContrib)[(size_t)slot * kNumLambda + wl];
+            if (cw == 0.0f) return false;
             const uint32_t p = st.cPath[slot];
             if (!sc.medium.present) {
                 addConnectionWl(st, st.cTarget[slot], p, wl, cw);
-                continue;
+                return false;
             }
             const float4 o = st.cRay[2 * (size_t)slot], d = st.cRay[2 * (size_t)slot + 1];
-            const Rng rng{mix64(keyOf(st, p) ^ (0x9e3779b97f4a7c15ull * (st.cMeta[slot] + 1))), (uint32_t)wl << 24};
+            const uint64_t key = mix64(keyOf(st, p) ^ (0x9e3779b97f4a7c15ull * (st.cMeta[slot] + 1)));
             const float sig = evalSpectrumAt(sc, sc.medium.sigmaE, lambdaAt(wl, st.wlOffset[p]));
-            walking = trBegin(sc.medium, q, xyz(o), xyz(d), o.w, d.w, sig, true, rng);
-            if (!walking) addConnectionWl(st, st.cTarget[slot], p, wl, cw * q.T);
-        }
-        if (!__any_sync(0xffffffffu, walking)) break;
-        if (walking) {
-            walking = trStep(sc.medium, q);
-            if (!walking) addConnectionWl(st, st.cTarget[slot], st.cPath[slot], wl, cw * q.T);
-        }
-    }
+            if (trBegin(sc.medium, q, xyz(o), xyz(d), o.w, d.w, sig, true, key, (uint32_t)wl << 24)) return true;
+            addConnectionWl(st, st.cTarget[slot], p, wl, cw * q.T);
+            return false;
+        },
+        [&](uint32_t item, const TrWalk &q) {
+            const uint32_t slot = st.mQueue[item / kNumLambda];
+            const int wl = (int)(item % kNumLambda);
+            const float cw = reinterpret_cast<const float*>(st.cContrib)[(size_t)slot * kNumLambda + wl];
+            addConnectionWl(st, st.cTarget[slot], st.cPath[slot], wl, cw * q.T);
+        });
 }
 
 // The wave's contributions into the compensated film: per pixel, the sums of

@@ -1407,22 +1407,9 @@ __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kShadowVolMediu
         waveEnd(true);
         return;
     }
-    uint32_t poolNext = 0, poolEnd = 0;
-    TrWalk q;
-    uint32_t item = 0;
-    bool walking = false, exhausted = false;
-    for (;;) {
-        // lanes without a walk take items until theirs needs steps
-        for (;;) {
-            const bool need = !walking && !exhausted;
-            if (!__any_sync(0xffffffffu, need)) break;
-            const uint32_t it = trTake(need, take, poolNext, poolEnd);
-            if (!need) continue;
-            if (it >= n) {
-                exhausted = true;
-                continue;
-            }
-            item = it;
+    trRun(
+        sc.medium, n, take,
+        [&](uint32_t item, TrWalk &q) {
             const uint32_t p = queue[item / kNumLambda];
             const int wl = (int)(item % kNumLambda);
             const float4 o = ws.shRay[2 * (size_t)p], d = ws.shRay[2 * (size_t)p + 1];
@@ -1431,23 +1418,18 @@ __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kShadowVolMediu
             const bool wlSelected = (info & kInfoWlSelected) != 0;
             // this thread's wavelength only, with the shading kernel's arithmetic
             const float sig = evalSpectrumAt(sc, sc.medium.sigmaE, lambdaAt(wl, ws.ps[p].wlOffset));
-            const Rng rng{mix64(loadKey(ws, p) ^ (0x9e3779b97f4a7c15ull * (bounce + 1))), (uint32_t)wl << 24};
-            walking = trBegin(sc.medium, q, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}, o.w, d.w, sig,
-                              !wlSelected || wl == sel, rng);
-            if (!walking && q.T != 0.0f) {
-                const size_t k = (size_t)p * kNumLambda + wl;
-                ws.L[k] += q.T * ws.shContrib[k];
-            }
-        }
-        if (!__any_sync(0xffffffffu, walking)) break;
-        if (walking) {
-            walking = trStep(sc.medium, q);
-            if (!walking && q.T != 0.0f) {
-                const size_t k = (size_t)queue[item / kNumLambda] * kNumLambda + item % kNumLambda;
-                ws.L[k] += q.T * ws.shContrib[k];
-            }
-        }
-    }
+            if (trBegin(sc.medium, q, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}, o.w, d.w, sig, !wlSelected || wl == sel,
+                        mix64(loadKey(ws, p) ^ (0x9e3779b97f4a7c15ull * (bounce + 1))), (uint32_t)wl << 24))
+                return true;
+            const size_t k = (size_t)p * kNumLambda + wl;
+            if (q.T != 0.0f) ws.L[k] += q.T * ws.shContrib[k];
+            return false;
+        },
+        [&](uint32_t item, const TrWalk &q) {
+            if (q.T == 0.0f) return;
+            const size_t k = (size_t)queue[item / kNumLambda] * kNumLambda + item % kNumLambda;
+            ws.L[k] += q.T * ws.shContrib[k];
+        });
     waveEnd(true);
 }
 
