@@ -634,10 +634,11 @@ int slrgpu_film_to_bmp(const float* film, uint32_t width, uint32_t height, int f
     if (!film) return fail(SLRGPU_ERR_INVALID_ARGUMENT, "film is NULL");
     if (width == 0 || height == 0) return fail(SLRGPU_ERR_INVALID_ARGUMENT, "width and height must be positive");
     const uint32_t rowBytes = 3 * width + width % 4;
-    std::vector<uint8_t> buf((size_t)rowBytes * height);
-    int rc = filmToBmp(film, width, height, film_on_device != 0, scale, sensitivity, buf.data());
+    const size_t rowsBytes = (size_t)rowBytes * height;
+    std::vector<uint8_t> buf(pixels ? 0 : rowsBytes);   // straight into the caller's array where there is one
+    uint8_t* rows = pixels ? pixels : buf.data();
+    int rc = filmToBmp(film, width, height, film_on_device != 0, scale, sensitivity, rows);
     if (rc != SLRGPU_OK) return rc;
-    if (pixels) std::memcpy(pixels, buf.data(), buf.size());
     if (path) {
         // 54-byte BITMAPFILEHEADER + BITMAPINFOHEADER, 24 bits, no compression,
         // 1 pixel per metre (Helper/bmp_exporter.cpp:15-53).
@@ -647,7 +648,7 @@ int slrgpu_film_to_bmp(const float* film, uint32_t width, uint32_t height, int f
         auto put16 = [&](int off, uint16_t v) { header[off] = (uint8_t)v; header[off + 1] = (uint8_t)(v >> 8); };
         header[0] = 'B';
         header[1] = 'M';
-        put32(2, (uint32_t)buf.size() + 54);
+        put32(2, (uint32_t)rowsBytes + 54);
         put32(10, 54);
         put32(14, 40);
         put32(18, width);
@@ -655,13 +656,13 @@ int slrgpu_film_to_bmp(const float* film, uint32_t width, uint32_t height, int f
         put16(26, 1);
         put16(28, 24);
         put32(30, 0);
-        put32(34, (uint32_t)buf.size());
+        put32(34, (uint32_t)rowsBytes);
         put32(38, 1);
         put32(42, 1);
         FILE* fp = std::fopen(path, "wb");
         if (!fp) return fail(SLRGPU_ERR_INVALID_ARGUMENT, std::string("cannot open ") + path);
         bool ok = std::fwrite(header, 1, sizeof(header), fp) == sizeof(header) &&
-                  std::fwrite(buf.data(), 1, buf.size(), fp) == buf.size();
+                  std::fwrite(rows, 1, rowsBytes, fp) == rowsBytes;
         std::fclose(fp);
         if (!ok) return fail(SLRGPU_ERR_INVALID_ARGUMENT, std::string("cannot write ") + path);
     }
