@@ -14,9 +14,10 @@
 // GPU structure, one wave at a time:
 //   kBptInit     one thread per path: pixel and wavelengths, the light vertex
 //                and the lens vertex, the first ray of each subpath;
-//   kBptBounce   per bounce, over the queue of live subpaths (both kinds
-//                mixed): closest hit, vertex creation, implicit emission,
-//                BSDF sampling with reverse densities, Russian roulette;
+//   kBptExtend   per bounce, over the queue of live subpaths (both kinds
+//                mixed): the closest hit;
+//   kBptBounce   the same subpaths: vertex creation, implicit emission, BSDF
+//                sampling with reverse densities, Russian roulette;
 //   kBptConnect  one thread per eye vertex: the connections with every light
 //                vertex of its path (shadow ray, MIS weight, contribution);
 //   kBptAccumulate  per pixel: the wave's per-path sums and the splat film
@@ -92,6 +93,7 @@ struct BptState {
     float4* bsdfA;        // [(D + 1) * S * 4] first spectrum of a surface vertex's BSDF
     float4* rayOrg;       // [S] xyz, tmin
     float4* rayDir;       // [S]
+    float4* hit;          // [S] t, b1, b2, primitive bits of the bounce's closest hit
     float4* alphaPend;    // [S * 4] throughput arriving at the next vertex
     float4* aux;          // [S] dirPdf, cosLast, rrPend, info bits
     uint32_t* rngCounter; // [S]
@@ -114,9 +116,10 @@ struct BptState {
     uint32_t* cPath;      // [connCap] path of the connection (volumetric: wavelengths, RNG key)
     uint32_t* cMeta;      // [connCap] eye vertex index << 8 | light vertex number (volumetric RNG stream)
     uint32_t* mQueue;     // [connCap] unoccluded connections whose transmittance is due (volumetric)
-    uint32_t* counters;   // [D + 5] queue sizes per bounce, eye vertices to connect, queued
+    uint32_t* counters;   // [2D + 6] queue sizes per bounce, eye vertices to connect, queued
                           // connections, connections waiting for their transmittance, the
-                          // transmittance kernel's work counter
+                          // work counters of the transmittance and shadow kernels and of
+                          // each bounce's closest hits
     unsigned long long* stats;   // 0 extension rays, 1 shadow rays, 2 dropped contributions
 };
 
@@ -489,11 +492,51 @@ __device__ __forceinline__ float vertexCos(const BptGeom &g, uint32_t flags, V3 
     return ((flags >> kVfKindShift) & 3u) == kVtxMedium ? 1.0f : absDot(d, xyz(g.ng));
 }
 
+// Closest hits of the bounce's subpaths, with the dynamic ray fetch of the path
+// tracer's extension kernel.  Apart from the bounce kernel, whose 128
+// registers leave 16 warps an SM, the walks have 32 to hide their node fetches.
+__global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kBptExtend(DevScene sc, BptState st,
+                                                                         const uint32_t* __restrict__ queue,
+                                                                         const uint32_t* __restrict__ count,
+                                                                         uint32_t* cursor) {
+    __shared__ StackEntry shared[kSharedStackEntries * 256];
+    const uint32_t n = *count;
+    const float inf = __int_as_float(0x7f800000);
+    ClosestStack stack(shared);
+    ClosestWalk<false> walk;
+    uint32_t sp = 0;
+    bool live = false, drained = false;
+    for (;;) {
+        uint32_t slot;
+        bool fin = false;
+        if (refillLanes(live, cursor, n, drained, &slot)) {
+            sp = queue[slot];
+            const float4 ro = st.rayOrg[sp], rd = st.rayDir[sp];
+            fin = walk.begin(sc, xyz(ro), xyz(rd), ro.w, inf);
+            live = true;
+        }
+        if (live && !fin) fin = walk.advance(sc, stack, SLRGPU_TRACE_REFILL_VISITS);
+        if (live && fin) {
+            st.hit[sp] = make_float4(walk.hit.t, walk.hit.b1, walk.hit.b2, __uint_as_float(walk.hit.prim));
+            live = false;
+        }
+        if (drained && !__any_sync(0xffffffffu, live)) return;
+    }
+}
+
 // One bounce of every live subpath: generateSubPath's loop body
-// (BPTRenderer.cpp:304-379; VOL: VolumetricBPTRenderer.cpp:311-391, where
+// (BPTRenderer.cpp:304-379) behind its closest hit (kBptExtend; VOL: VolumetricBPTRenderer.cpp:311-391, where
 // Scene::interact may stop the ray at a scattering point in the medium).  A
-// subpath holds at most D + 1 vertices.
-template <bool VOL>
+// subpath holds at most D + 1 vertices.  K: the kind of every material of the
+// scene, whose BSDF is then compiled in alone (no run-time dispatch, no calls,
+// its spectra in registers), or -1.  On the box at 512 x 512 x 4 (16 vertices a
+// subpath) the closest hits and bounces go from 2.9 to 2.0 ms and the
+// connections from 3.85 to 2.55 ms, the frame from 7.9 to 5.8 ms; 3 or 4
+// blocks per SM (80, 64 registers, 550 B of spills and up) 5.96 and 6.1 ms.
+// The volumetric instance is compiled for
+// any material only: with one kind its collision distances come out an ulp
+// apart, which makes other paths of a few.
+template <bool VOL, int K>
 __global__ void __launch_bounds__(256, 2) kBptBounce(DevScene sc, BptState st, const uint32_t* __restrict__ inQueue,
                                                      const uint32_t* __restrict__ inCount, uint32_t* outQueue,
                                                      uint32_t* outCount) {
@@ -523,8 +566,8 @@ __global__ void __launch_bounds__(256, 2) kBptBounce(DevScene sc, BptState st, c
             Rng rng{keyOf(st, p), st.rngCounter[sp]};
             Spec alpha;
             loadAlpha(st.alphaPend, sp, alpha);
-            Hit h;
-            traceClosest(sc, org, dir, ro.w, inf, &h);
+            const float4 hv = st.hit[sp];
+            const Hit h{hv.x, hv.y, hv.z, __float_as_uint(hv.w)};
             // Scene::interact (Scene.cpp:66-94): a collision in the medium
             // before the surface, with the medium throughput on the way.
             bool medHit = false;
@@ -643,7 +686,8 @@ __global__ void __launch_bounds__(256, 2) kBptBounce(DevScene sc, BptState st, c
                     for (int q = 0; q < kNumLambda; ++q)
                         B.a.v[q] = (in && sigmaE.v[q] > 0) ? sigmaS.v[q] / sigmaE.v[q] : 0.0f;
                 } else {
-                    makeBsdf(sc, mat, lambdas, wlSelected, B);
+                    if (K < 0) makeBsdf(sc, mat, lambdas, wlSelected, B);
+                    else makeBsdfK<(K < 0 ? 0 : K)>(sc, mat, (const float*)lambdas, wlSelected, B);
                 }
                 storeAlpha(st.bsdfA, vi, B.a);   // the connections reuse it (Lambert reflectance, albedo)
                 // Implicit path, no light subpath vertex (BPTRenderer.cpp:318-340).
@@ -691,7 +735,7 @@ __global__ void __launch_bounds__(256, 2) kBptBounce(DevScene sc, BptState st, c
                     } else {
                         RevQuery q{dirOut, gnl, sel, adjoint};
                         const float uc = rng.next(), u0 = rng.next(), u1 = rng.next();
-                        bsdfSampleRev(B, q, uc, u0, u1, &bs, fs, &revPdf, revFs);
+                        bsdfSampleRev<K>(B, q, uc, u0, u1, &bs, fs, &revPdf, revFs);
                     }
                     if (bs.pdf != 0.0f && !specIsZero(fs)) {
                         if ((bs.type & kDirDispersive) && !wlSelected) wlSelected = true;
@@ -732,9 +776,10 @@ __global__ void __launch_bounds__(256, 2) kBptBounce(DevScene sc, BptState st, c
 
 // The BSDF of a surface vertex for its connections: Lambert from the
 // reflectance cached at the vertex, other kinds evaluated again.
+template <int K>
 __device__ __forceinline__ void vertexBsdf(const DevScene &sc, const BptState &st, size_t vi, uint32_t material,
                                            uint32_t flags, const float* lambdas, Bsdf &B) {
-    if (((flags >> kVfMatShift) & 0xfu) == kMatMatte) {
+    if (K == (int)kMatMatte || ((flags >> kVfMatShift) & 0xfu) == kMatMatte) {
         B.kind = kMatMatte;
         B.ax = B.ay = 0.0f;
         B.dispersive = (flags & kVfWlSelected) == 0;
@@ -752,7 +797,7 @@ __device__ __forceinline__ void vertexBsdf(const DevScene &sc, const BptState &s
 // or pixel | kTargetSplat when it lands through the lens (t = 1).  Without
 // a medium the splat contribution comes binned into film bins; VOL leaves it
 // per wavelength for the transmittance.
-template <bool VOL>
+template <bool VOL, int K>
 __device__ bool connectOne(const DevScene &sc, const BptState &st, uint32_t evi, uint32_t s, uint32_t width,
                            uint32_t height, float4* rayOrg, float4* rayDir, Spec &c, uint32_t* target,
                            bool* dropped) {
@@ -808,10 +853,10 @@ __device__ bool connectOne(const DevScene &sc, const BptState &st, uint32_t evi,
         lRev = lDDF;
     } else {
         Bsdf lB;
-        vertexBsdf(sc, st, lvi, __float_as_uint(lg.pg.w), lpd.flags, lambdas, lB);
+        vertexBsdf<K>(sc, st, lvi, __float_as_uint(lg.pg.w), lpd.flags, lambdas, lB);
         RevQuery lq{V3{lg.nz.w, lg.tx.w, lg.ng.w}, lF.toLocal(xyz(lg.ng)), sel, true};
-        bsdfEvalRev(lB, lq, lc, lDDF, lRev);
-        lExt1DirPdf = bsdfPdfRev(lB, lq, lc, &eExt2DirPdf);
+        bsdfEvalRev<K>(lB, lq, lc, lDDF, lRev);
+        lExt1DirPdf = bsdfPdfRev<K>(lB, lq, lc, &eExt2DirPdf);
     }
     // eye end: importance of the lens, the BSDF or the medium's
     const V3 ec = eF.toLocal(cv);
@@ -831,10 +876,10 @@ __device__ bool connectOne(const DevScene &sc, const BptState &st, uint32_t evi,
         eRev = eDDF;
     } else {
         Bsdf eB;
-        vertexBsdf(sc, st, evi, __float_as_uint(eg.pg.w), ep.flags, lambdas, eB);
+        vertexBsdf<K>(sc, st, evi, __float_as_uint(eg.pg.w), ep.flags, lambdas, eB);
         RevQuery eq{V3{eg.nz.w, eg.tx.w, eg.ng.w}, eF.toLocal(xyz(eg.ng)), sel, false};
-        bsdfEvalRev(eB, eq, ec, eDDF, eRev);
-        eExt1DirPdf = bsdfPdfRev(eB, eq, ec, &lExt2DirPdf);
+        bsdfEvalRev<K>(eB, eq, ec, eDDF, eRev);
+        eExt1DirPdf = bsdfPdfRev<K>(eB, eq, ec, &lExt2DirPdf);
     }
     Spec ct;
     bool nz = false;
@@ -952,7 +997,7 @@ __device__ __forceinline__ void addConnectionWl(const BptState &st, uint32_t tar
 // lane one (eye vertex, light vertex) pair per round, so lanes stay busy
 // whatever the subpath lengths.  Connections that contribute go to the
 // shadow queue.
-template <bool VOL>
+template <bool VOL, int K>
 __global__ void __launch_bounds__(256, 2) kBptConnect(DevScene sc, BptState st, uint32_t width, uint32_t height,
                                                       const uint32_t* __restrict__ queue,
                                                       const uint32_t* __restrict__ count, uint32_t first,
@@ -998,7 +1043,7 @@ __global__ void __launch_bounds__(256, 2) kBptConnect(DevScene sc, BptState st, 
             uint32_t target = 0;
             if (j < total) {
                 bool drop;
-                push = connectOne<VOL>(sc, st, ev, sIdx, width, height, &ro, &rd, c, &target, &drop);
+                push = connectOne<VOL, K>(sc, st, ev, sIdx, width, height, &ro, &rd, c, &target, &drop);
                 dropped += drop ? 1 : 0;
             }
             const unsigned mask = __ballot_sync(full, push);
@@ -1028,14 +1073,25 @@ __global__ void __launch_bounds__(256, 2) kBptConnect(DevScene sc, BptState st, 
 template <bool VOL>
 __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kBptShadow(DevScene sc, BptState st,
                                                                          const uint32_t* __restrict__ shCount,
-                                                                         uint32_t* medCount) {
+                                                                         uint32_t* medCount, uint32_t* cursor) {
     const uint32_t n = min(*shCount, st.connCap);
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        bool pushMedium = false;
-        if (i < n) {
+    LocalStack<uint32_t> stack;
+    AnyWalk<false> walk;
+    uint32_t i = 0;
+    bool live = false, drained = false;
+    for (;;) {
+        uint32_t slot;
+        bool fin = false;
+        if (refillLanes(live, cursor, n, drained, &slot)) {
+            i = slot;
             const float4 o = st.cRay[2 * (size_t)i], d = st.cRay[2 * (size_t)i + 1];
-            if (!traceAny(sc, xyz(o), xyz(d), o.w, d.w)) {
+            fin = walk.begin(sc, xyz(o), xyz(d), o.w, d.w);
+            live = true;
+        }
+        if (live && !fin) fin = walk.advance(sc, stack, SLRGPU_TRACE_REFILL_VISITS);
+        bool pushMedium = false;
+        if (live && fin) {
+            if (!walk.occluded) {
                 if (VOL) {
                     pushMedium = true;
                 } else {
@@ -1044,8 +1100,10 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kBptShadow(DevSc
                     addConnection(st, st.cTarget[i], c);
                 }
             }
+            live = false;
         }
-        if (VOL) queuePush(st.mQueue, medCount, i, pushMedium);
+        if (VOL && __any_sync(0xffffffffu, pushMedium)) queuePush(st.mQueue, medCount, i, pushMedium);
+        if (drained && !__any_sync(0xffffffffu, live)) break;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&st.stats[1], (unsigned long long)n);
 }
@@ -1146,7 +1204,8 @@ int gridFor(const void* kernel, int block) {
 }
 
 struct BptGrids {
-    int init[2], bounce[2], connect[2], shadow[2], medium, accumulate;
+    // [VOL], and [VOL][scene of Lambert materials alone]
+    int init[2], bounce[2][2], connect[2][2], shadow[2], medium, accumulate, extend;
 };
 const BptGrids &bptGrids() {
     static BptGrids g;
@@ -1154,10 +1213,14 @@ const BptGrids &bptGrids() {
     std::call_once(once, [&]() {
         g.init[0] = gridFor((const void*)kBptInit<false>, 256);
         g.init[1] = gridFor((const void*)kBptInit<true>, 256);
-        g.bounce[0] = gridFor((const void*)kBptBounce<false>, 256);
-        g.bounce[1] = gridFor((const void*)kBptBounce<true>, 256);
-        g.connect[0] = gridFor((const void*)kBptConnect<false>, 256);
-        g.connect[1] = gridFor((const void*)kBptConnect<true>, 256);
+        g.extend = gridFor((const void*)kBptExtend, 256);
+        g.bounce[0][0] = gridFor((const void*)kBptBounce<false, -1>, 256);
+        g.bounce[0][1] = gridFor((const void*)kBptBounce<false, kMatMatte>, 256);
+        g.bounce[1][0] = gridFor((const void*)kBptBounce<true, -1>, 256);
+        g.connect[0][0] = gridFor((const void*)kBptConnect<false, -1>, 256);
+        g.connect[0][1] = gridFor((const void*)kBptConnect<false, kMatMatte>, 256);
+        g.connect[1][0] = gridFor((const void*)kBptConnect<true, -1>, 256);
+        g.connect[1][1] = gridFor((const void*)kBptConnect<true, kMatMatte>, 256);
         g.shadow[0] = gridFor((const void*)kBptShadow<false>, 256);
         g.shadow[1] = gridFor((const void*)kBptShadow<true>, 256);
         g.medium = gridFor((const void*)kVbptMedium, 256);
@@ -1215,7 +1278,7 @@ struct BptEngine {
         bool ok = (s.geom = alloc<BptGeom>(V, &e)) && (s.pdf = alloc<BptPdf>(V, &e)) &&
                   (s.alpha = alloc<float4>(V * 4, &e)) && (s.bsdfA = alloc<float4>(V * 4, &e)) &&
                   (s.rayOrg = alloc<float4>(S, &e)) &&
-                  (s.rayDir = alloc<float4>(S, &e)) && (s.alphaPend = alloc<float4>(S * 4, &e)) &&
+                  (s.rayDir = alloc<float4>(S, &e)) && (s.hit = alloc<float4>(S, &e)) && (s.alphaPend = alloc<float4>(S * 4, &e)) &&
                   (s.aux = alloc<float4>(S, &e)) && (s.rngCounter = alloc<uint32_t>(S, &e)) &&
                   (s.numVerts = alloc<uint32_t>(S, &e)) && (s.rngKey = alloc<uint2>(N, &e)) &&
                   (s.pix = alloc<float2>(N, &e)) && (s.wlOffset = alloc<float>(N, &e)) &&
@@ -1229,7 +1292,7 @@ struct BptEngine {
                   (s.cPath = alloc<uint32_t>((size_t)kConnPerPath * N, &e)) &&
                   (s.cMeta = alloc<uint32_t>((size_t)kConnPerPath * N, &e)) &&
                   (s.mQueue = alloc<uint32_t>((size_t)kConnPerPath * N, &e)) &&
-                  (s.counters = alloc<uint32_t>(D + 5, &e)) && (s.stats = alloc<unsigned long long>(4, &e));
+                  (s.counters = alloc<uint32_t>(2 * D + 6, &e)) && (s.stats = alloc<unsigned long long>(4, &e));
         if (!ok) {
             release();
             setError(std::string("bidirectional path state allocation failed: ") + cudaGetErrorString(e));
@@ -1255,7 +1318,7 @@ void bptEngineDestroy(BptEngine* e) { delete e; }
 
 uint64_t bptStateBytesPerPath(uint32_t maxDepth) {
     const uint64_t V = 2ull * (maxDepth + 1);
-    return V * (sizeof(BptGeom) + sizeof(BptPdf) + 128) + 2 * (16 + 16 + 64 + 16 + 4 + 4) + 8 + 8 + 4 + 4 +
+    return V * (sizeof(BptGeom) + sizeof(BptPdf) + 128) + 2 * (16 + 16 + 16 + 64 + 16 + 4 + 4) + 8 + 8 + 4 + 4 +
            4 * kNumLambda + 8 + 4ull * (maxDepth + 1) + kConnPerPath * (32 + 64 + 16);
 }
 
@@ -1272,6 +1335,7 @@ int renderBpt(BptEngine &eng, const DeviceScene &ds, const slrgpu_settings &s, f
         return SLRGPU_ERR_INVALID_ARGUMENT;
     }
     const uint32_t D = s.max_depth;
+    const bool lambert = ds.kindMask == 1u << kMatMatte;   // every material is Lambertian
     const uint32_t gridW = (s.width + 7) / 8 * 8, gridH = (s.height + 7) / 8 * 8;
     const uint32_t G = gridW * gridH;
     const uint64_t perPath = bptStateBytesPerPath(D);
@@ -1331,22 +1395,28 @@ int renderBpt(BptEngine &eng, const DeviceScene &ds, const slrgpu_settings &s, f
         wv.samples = std::min(S, s.spp - base);
         wv.seed = s.seed;
         wv.numPaths = wv.samples * G;
-        cudaMemsetAsync(st.counters, 0, (D + 5) * sizeof(uint32_t), stream);
+        cudaMemsetAsync(st.counters, 0, (2 * D + 6) * sizeof(uint32_t), stream);
         mark(SLRGPU_KERNEL_RAYGEN);
         if (vol) kBptInit<true><<<g.init[1], 256, 0, stream>>>(ds.sc, st, wv);
         else kBptInit<false><<<g.init[0], 256, 0, stream>>>(ds.sc, st, wv);
         markEnd();
         ++nl;
         for (uint32_t b = 0; b < D; ++b) {
+            const uint32_t* inQueue = st.queue[b & 1];
+            uint32_t* outQueue = st.queue[(b + 1) & 1];
+            const uint32_t* inCount = st.counters + b;
             mark(SLRGPU_KERNEL_EXTEND);
-            if (vol)
-                kBptBounce<true><<<g.bounce[1], 256, 0, stream>>>(ds.sc, st, st.queue[b & 1], st.counters + b,
-                                                                   st.queue[(b + 1) & 1], st.counters + b + 1);
-            else
-                kBptBounce<false><<<g.bounce[0], 256, 0, stream>>>(ds.sc, st, st.queue[b & 1], st.counters + b,
-                                                                    st.queue[(b + 1) & 1], st.counters + b + 1);
+            kBptExtend<<<g.extend, 256, 0, stream>>>(ds.sc, st, inQueue, inCount, st.counters + D + 6 + b);
             markEnd();
-            ++nl;
+            mark(SLRGPU_KERNEL_EXTEND);
+#define SLRGPU_BPT_BOUNCE(V, KK) \
+    kBptBounce<V, KK><<<g.bounce[V][KK == (int)kMatMatte], 256, 0, stream>>>(ds.sc, st, inQueue, inCount, outQueue, st.counters + b + 1)
+            if (vol) SLRGPU_BPT_BOUNCE(true, -1);
+            else if (lambert) SLRGPU_BPT_BOUNCE(false, kMatMatte);
+            else SLRGPU_BPT_BOUNCE(false, -1);
+#undef SLRGPU_BPT_BOUNCE
+            markEnd();
+            nl += 2;
         }
         // Connections in passes of at most connCap / (D + 1) eye vertices:
         // each has at most D + 1 light vertices to connect to, so a pass
@@ -1361,24 +1431,24 @@ int renderBpt(BptEngine &eng, const DeviceScene &ds, const slrgpu_settings &s, f
         }
         const uint32_t perPass = std::max(1u, st.connCap / (D + 1));
         for (uint32_t first = 0; first < items; first += perPass) {
-            cudaMemsetAsync(st.counters + D + 2, 0, 3 * sizeof(uint32_t), stream);
+            cudaMemsetAsync(st.counters + D + 2, 0, 4 * sizeof(uint32_t), stream);
             mark(SLRGPU_KERNEL_SHADE);
-            if (vol)
-                kBptConnect<true><<<g.connect[1], 256, 0, stream>>>(ds.sc, st, s.width, s.height, st.connQueue,
-                                                                     st.counters + D + 1, first, perPass,
-                                                                     st.counters + D + 2);
-            else
-                kBptConnect<false><<<g.connect[0], 256, 0, stream>>>(ds.sc, st, s.width, s.height, st.connQueue,
-                                                                      st.counters + D + 1, first, perPass,
-                                                                      st.counters + D + 2);
+#define SLRGPU_BPT_CONNECT(V, KK)                                                                                  \
+    kBptConnect<V, KK><<<g.connect[V][KK == (int)kMatMatte], 256, 0, stream>>>(                                    \
+        ds.sc, st, s.width, s.height, st.connQueue, st.counters + D + 1, first, perPass, st.counters + D + 2)
+            if (vol && lambert) SLRGPU_BPT_CONNECT(true, kMatMatte);
+            else if (vol) SLRGPU_BPT_CONNECT(true, -1);
+            else if (lambert) SLRGPU_BPT_CONNECT(false, kMatMatte);
+            else SLRGPU_BPT_CONNECT(false, -1);
+#undef SLRGPU_BPT_CONNECT
             markEnd();
             mark(SLRGPU_KERNEL_SHADOW);
             if (vol)
                 kBptShadow<true><<<g.shadow[1], 256, 0, stream>>>(ds.sc, st, st.counters + D + 2,
-                                                                   st.counters + D + 3);
+                                                                   st.counters + D + 3, st.counters + D + 5);
             else
                 kBptShadow<false><<<g.shadow[0], 256, 0, stream>>>(ds.sc, st, st.counters + D + 2,
-                                                                    st.counters + D + 3);
+                                                                    st.counters + D + 3, st.counters + D + 5);
             markEnd();
             nl += 2;
             if (vol) {

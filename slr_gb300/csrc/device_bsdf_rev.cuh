@@ -28,15 +28,16 @@ __device__ __forceinline__ float snCorrection(const RevQuery &q, V3 other) {
 // Sampling (basic_bsdfs.cpp:13-153, microfacet_bsdfs.cpp:11-211).  res->pdf
 // == 0 on failure; on success fs and revFs carry the shading-normal
 // correction.
-static __device__ __noinline__ void bsdfSampleRev(const Bsdf &B, const RevQuery &q, float uc, float u0, float u1,
-                                           BsdfSample* res, Spec &fs, float* revPdf, Spec &revFs) {
+template <int K>
+__device__ __forceinline__ void bsdfSampleRevBody(const Bsdf &B, const RevQuery &q, float uc, float u0, float u1,
+                                                  BsdfSample* res, Spec &fs, float* revPdf, Spec &revFs) {
     res->pdf = 0.0f;
     res->type = 0;
     res->dir = V3{0, 0, 1};
     *revPdf = 0.0f;
     fs = specConst(0.0f);
     revFs = specConst(0.0f);
-    switch (B.kind) {
+    switch (K < 0 ? B.kind : (uint32_t)K) {
     case kMatMatte: {
         V3 d = cosineSampleHemisphere(u0, u1);
         res->pdf = d.z * kInvPiF;
@@ -186,9 +187,10 @@ static __device__ __noinline__ void bsdfSampleRev(const Bsdf &B, const RevQuery 
 }
 
 // Evaluation with the reverse value (basic_bsdfs.cpp:28-39, microfacet_bsdfs.cpp:48-72, 213-265).
-static __device__ __noinline__ void bsdfEvalRev(const Bsdf &B, const RevQuery &q, V3 dir, Spec &fs, Spec &revFs) {
+template <int K>
+__device__ __forceinline__ void bsdfEvalRevBody(const Bsdf &B, const RevQuery &q, V3 dir, Spec &fs, Spec &revFs) {
     fs = specConst(0.0f);
-    switch (B.kind) {
+    switch (K < 0 ? B.kind : (uint32_t)K) {
     case kMatMatte:
         if (q.dir.z * dir.z > 0.0f) specScale(B.a, 1.0f / kPiF, fs);
         break;
@@ -238,9 +240,10 @@ static __device__ __noinline__ void bsdfEvalRev(const Bsdf &B, const RevQuery &q
 }
 
 // Density with the reverse density (basic_bsdfs.cpp:41-50, microfacet_bsdfs.cpp:74-102, 267-318).
-static __device__ __noinline__ float bsdfPdfRev(const Bsdf &B, const RevQuery &q, V3 dir, float* revPdf) {
+template <int K>
+__device__ __forceinline__ float bsdfPdfRevBody(const Bsdf &B, const RevQuery &q, V3 dir, float* revPdf) {
     *revPdf = 0.0f;
-    switch (B.kind) {
+    switch (K < 0 ? B.kind : (uint32_t)K) {
     case kMatMatte:
         if (q.dir.z * dir.z <= 0.0f) return 0.0f;
         *revPdf = fabsf(q.dir.z) * kInvPiF;
@@ -285,6 +288,35 @@ static __device__ __noinline__ float bsdfPdfRev(const Bsdf &B, const RevQuery &q
     default:
         return 0.0f;
     }
+}
+
+// K < 0: any material, dispatched at run time and kept out of line; K >= 0:
+// that kind alone, inlined.
+static __device__ __noinline__ void bsdfSampleRevAny(const Bsdf &B, const RevQuery &q, float uc, float u0, float u1,
+                                                     BsdfSample* res, Spec &fs, float* revPdf, Spec &revFs) {
+    bsdfSampleRevBody<-1>(B, q, uc, u0, u1, res, fs, revPdf, revFs);
+}
+static __device__ __noinline__ void bsdfEvalRevAny(const Bsdf &B, const RevQuery &q, V3 dir, Spec &fs, Spec &revFs) {
+    bsdfEvalRevBody<-1>(B, q, dir, fs, revFs);
+}
+static __device__ __noinline__ float bsdfPdfRevAny(const Bsdf &B, const RevQuery &q, V3 dir, float* revPdf) {
+    return bsdfPdfRevBody<-1>(B, q, dir, revPdf);
+}
+template <int K>
+__device__ __forceinline__ void bsdfSampleRev(const Bsdf &B, const RevQuery &q, float uc, float u0, float u1,
+                                              BsdfSample* res, Spec &fs, float* revPdf, Spec &revFs) {
+    if (K < 0) bsdfSampleRevAny(B, q, uc, u0, u1, res, fs, revPdf, revFs);
+    else bsdfSampleRevBody<K>(B, q, uc, u0, u1, res, fs, revPdf, revFs);
+}
+template <int K>
+__device__ __forceinline__ void bsdfEvalRev(const Bsdf &B, const RevQuery &q, V3 dir, Spec &fs, Spec &revFs) {
+    if (K < 0) bsdfEvalRevAny(B, q, dir, fs, revFs);
+    else bsdfEvalRevBody<K>(B, q, dir, fs, revFs);
+}
+template <int K>
+__device__ __forceinline__ float bsdfPdfRev(const Bsdf &B, const RevQuery &q, V3 dir, float* revPdf) {
+    if (K < 0) return bsdfPdfRevAny(B, q, dir, revPdf);
+    return bsdfPdfRevBody<K>(B, q, dir, revPdf);
 }
 
 }  // namespace slrgpu

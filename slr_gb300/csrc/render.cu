@@ -306,45 +306,11 @@ __global__ void kRaygen(DevScene scArg, WaveState ws, const __grid_constant__ Wa
 #ifndef SLRGPU_TRACE_REFILL
 #define SLRGPU_TRACE_REFILL 1
 #endif
-#ifndef SLRGPU_TRACE_REFILL_LANES
-#define SLRGPU_TRACE_REFILL_LANES 8
-#endif
-#ifndef SLRGPU_TRACE_REFILL_VISITS
-#define SLRGPU_TRACE_REFILL_VISITS 16
-#endif
-static_assert(SLRGPU_TRACE_REFILL_LANES >= 1 && SLRGPU_TRACE_REFILL_LANES <= 32, "a warp has 32 lanes");
 // The same threshold for the ray-query kernel (slrgpu_trace_rays).
 #ifndef SLRGPU_QUERY_REFILL_LANES
 #define SLRGPU_QUERY_REFILL_LANES SLRGPU_TRACE_REFILL_LANES
 #endif
 static_assert(SLRGPU_QUERY_REFILL_LANES >= 1 && SLRGPU_QUERY_REFILL_LANES <= 32, "a warp has 32 lanes");
-
-// Stack entries of a closest-hit walk in shared memory: lanes at different
-// depths store to as many lines of local memory, but to different banks of
-// shared memory.  1,000,003 incoherent queries on 24k triangles 456 us without,
-// 448, 441, 440 and 441 with 4, 8, 12 and 16 entries.  The any-hit walk's
-// 4-byte entries stay local (4 Mi queries on 176k triangles 1528 us, 1557 with
-// 12 entries in shared memory: the L1 it takes counts for more).
-constexpr int kSharedStackEntries = 8;
-using ClosestStack = SharedStack<StackEntry, kSharedStackEntries>;
-
-// The refill step of a warp: when at least SLRGPU_TRACE_REFILL_LANES lanes
-// are idle and the queue is not drained, the idle lanes take the next queue
-// entries (*slot = entry index, or n when there is none left).  Returns
-// whether this lane got one.  Called by all 32 lanes.
-__device__ __forceinline__ bool refillLanes(bool live, uint32_t* cursor, uint32_t n, bool &drained, uint32_t* slot) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t idle = __ballot_sync(0xffffffffu, !live);
-    if (drained || (uint32_t)__popc(idle) < SLRGPU_TRACE_REFILL_LANES) return false;
-    const int leader = __ffs(idle) - 1;
-    uint32_t base = 0;
-    if ((int)lane == leader) base = atomicAdd(cursor, (uint32_t)__popc(idle));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    drained = base + (uint32_t)__popc(idle) >= n;
-    if (live) return false;
-    *slot = base + (uint32_t)__popc(idle & ((1u << lane) - 1));
-    return *slot < n;
-}
 
 // Shadow rays (PTRenderer.cpp:196-217): an unoccluded ray adds its stored
 // contribution to the path's radiance.
