@@ -1417,16 +1417,16 @@ __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kShadowVolMediu
 // Bound by the read of the paths' radiance and scalars (96 B a sample).  Four
 // lanes per pixel, each with four wavelengths and film bins: a sample's 64
 // bytes of radiance are one access of the quad, and a pixel's samples, which
-// lie next to each other, stream, eight of them loaded ahead of the sums'
+// lie next to each other, stream, four of them loaded ahead of the sums'
 // chain.  One thread per pixel took 0.42 ms on a 333 x 187 image with 24
 // samples, whose last pixel alone sums 576 (this kernel 0.23 ms), and sixteen
 // lanes repeated the per-sample work too often (1024 x 1024 x 64: 4.4 ms
-// against 1.8 ms, 3.5 TB/s).
+// against 1.8 ms, 3.5 TB/s; eight samples loaded ahead at 115 registers 2.3).
 // A render's first wave starts from zero sums without reading them, and its
 // last one writes the pixel-major film itself.
 constexpr uint32_t kFilmFirst = 1u;   // the film's sums start at zero: do not read them
 constexpr uint32_t kFilmKeep = 2u;    // store sums and compensations for a later wave
-__global__ void __launch_bounds__(256) kAccumulate(WaveState ws, const __grid_constant__ WaveParams wpArg,
+__global__ void __launch_bounds__(256, 3) kAccumulate(WaveState ws, const __grid_constant__ WaveParams wpArg,
                                                    const WaveParams* __restrict__ wpDev, uint32_t flags, float* out) {
     waveBegin(false);
     const WaveParams &wp = wpDev ? *wpDev : wpArg;
@@ -1460,7 +1460,7 @@ __global__ void __launch_bounds__(256) kAccumulate(WaveState ws, const __grid_co
         const uint32_t yEnd = y + 1 == sg.height ? sg.gridH : y + 1;
         const uint32_t n = sg.samples * (xEnd - x) * (yEnd - y);
         uint32_t s = 0, gx = x, gy = y;
-        constexpr uint32_t kAhead = 8;
+        constexpr uint32_t kAhead = 4;
         for (uint32_t i0 = 0; i0 < n; i0 += kAhead) {
             float4 Lv[kAhead];
             float w[kAhead], off[kAhead];
@@ -1552,33 +1552,44 @@ __global__ void kFilmToPixelMajor(const float* __restrict__ src, float* __restri
     }
 }
 
-// Ray queries (slrgpu_trace_rays): each warp takes the rays of its own
+// Ray queries (slrgpu_trace_rays): each block takes the rays of its own
 // contiguous range, and lanes whose walk has ended take the range's next rays
 // while the others go on walking (the refill of the wave kernels, with the
-// warp's cursor in registers instead of a counter in memory).
+// block's cursor in shared memory).  A range per warp left the block
+// waiting for its slowest warp (1,000,003 incoherent closest-hit queries on 24k
+// triangles 440 us against 400 now, 2 Mi coherent ones on 176k triangles 571
+// us at the start against 398).  Few rays
+// spread over the block's warps: no lane past `width` takes one.
 template <bool WT, bool ANY>
 __device__ __forceinline__ void traceQueries(const DevScene &sc, const float4* __restrict__ rays, uint32_t n,
-                                             uint32_t* prim, float* t, float* b1, float* b2, StackEntry* shared) {
+                                             uint32_t* prim, float* t, float* b1, float* b2, StackEntry* shared,
+                                             uint32_t* cursor) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t chunk = ((uint64_t)n + warps - 1) / warps;
-    const uint64_t first = (uint64_t)warp * chunk;
-    uint32_t cursor = first < n ? (uint32_t)first : n;
+    const uint64_t chunk = ((uint64_t)n + gridDim.x - 1) / gridDim.x;
+    const uint64_t first = (uint64_t)blockIdx.x * chunk;
     const uint32_t end = first + chunk < n ? (uint32_t)(first + chunk) : n;
+    if (threadIdx.x == 0) *cursor = first < n ? (uint32_t)first : n;
+    __syncthreads();
+    const uint32_t width = (uint32_t)min((chunk + 7) / 8, (uint64_t)32);
+    const uint32_t refill = min(width, (uint32_t)SLRGPU_QUERY_REFILL_LANES);
     ClosestStack cstack(shared);
     LocalStack<uint32_t> astack;
     ClosestWalk<WT> cw;
     AnyWalk<WT> aw;
     uint32_t i = 0;
-    bool live = false;
+    bool live = false, drained = false;
     for (;;) {
-        const uint32_t idle = __ballot_sync(0xffffffffu, !live);
+        const uint32_t idle = __ballot_sync(0xffffffffu, !live && lane < width);
         bool fin = false;
-        if (cursor < end && (uint32_t)__popc(idle) >= SLRGPU_QUERY_REFILL_LANES) {
-            if (!live) {
-                const uint32_t k = cursor + (uint32_t)__popc(idle & ((1u << lane) - 1));
-                if (k < end) {
+        if (!drained && (uint32_t)__popc(idle) >= refill) {
+            const int leader = __ffs(idle) - 1;
+            uint32_t base = 0;
+            if ((int)lane == leader) base = atomicAdd(cursor, (uint32_t)__popc(idle));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            drained = base >= end || end - base <= (uint32_t)__popc(idle);
+            if ((idle >> lane) & 1u) {
+                const uint32_t k = base + (uint32_t)__popc(idle & ((1u << lane) - 1));
+                if (base < end && k < end) {
                     i = k;
                     const float4 o = rays[2 * (size_t)i], d = rays[2 * (size_t)i + 1];
                     const V3 org = V3{o.x, o.y, o.z}, dir = V3{d.x, d.y, d.z};
@@ -1586,7 +1597,6 @@ __device__ __forceinline__ void traceQueries(const DevScene &sc, const float4* _
                     live = true;
                 }
             }
-            cursor = end - cursor > (uint32_t)__popc(idle) ? cursor + (uint32_t)__popc(idle) : end;
         }
         if (live && !fin)
             fin = ANY ? aw.advance(sc, astack, SLRGPU_TRACE_REFILL_VISITS)
@@ -1602,7 +1612,7 @@ __device__ __forceinline__ void traceQueries(const DevScene &sc, const float4* _
             }
             live = false;
         }
-        if (cursor >= end && !__any_sync(0xffffffffu, live)) return;
+        if (drained && !__any_sync(0xffffffffu, live)) return;
     }
 }
 
@@ -1610,13 +1620,14 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kTrace(DevScene 
                                                                      uint32_t n, int anyHit, uint32_t* prim, float* t,
                                                                      float* b1, float* b2) {
     __shared__ StackEntry shared[kSharedStackEntries * 256];
+    __shared__ uint32_t cursor;
     const float4* r = reinterpret_cast<const float4*>(rays);
     if (anyHit) {
-        if (sc.watertight) traceQueries<true, true>(sc, r, n, prim, t, b1, b2, shared);
-        else traceQueries<false, true>(sc, r, n, prim, t, b1, b2, shared);
+        if (sc.watertight) traceQueries<true, true>(sc, r, n, prim, t, b1, b2, shared, &cursor);
+        else traceQueries<false, true>(sc, r, n, prim, t, b1, b2, shared, &cursor);
     } else {
-        if (sc.watertight) traceQueries<true, false>(sc, r, n, prim, t, b1, b2, shared);
-        else traceQueries<false, false>(sc, r, n, prim, t, b1, b2, shared);
+        if (sc.watertight) traceQueries<true, false>(sc, r, n, prim, t, b1, b2, shared, &cursor);
+        else traceQueries<false, false>(sc, r, n, prim, t, b1, b2, shared, &cursor);
     }
 }
 
