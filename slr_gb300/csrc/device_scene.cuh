@@ -48,6 +48,31 @@ __device__ __forceinline__ void queuePush(uint32_t* queue, uint32_t* count, uint
     queue[base + __popc(mask & ((1u << lane) - 1))] = value;
 }
 
+// The reference's renderers sample the sensor in whole 8x8 tiles
+// (ImageSensor.cpp:13-14, :42-43; PTRenderer.cpp:104-110), also where a tile
+// hangs over the image's right or bottom edge; ImageSensor::add
+// (ImageSensor.cpp:125-130) clamps those samples into the last column / row.
+// A wave therefore traces every position of the tile-padded sample grid.
+constexpr uint32_t kSensorTile = 8;
+__host__ __device__ __forceinline__ uint32_t padToTile(uint32_t n) {
+    return (n + kSensorTile - 1) / kSensorTile * kSensorTile;
+}
+
+// The order in which waves walk the grid's positions: tile by tile, row by row
+// of tiles, Morton order inside a tile.
+__device__ __forceinline__ void tilePosition(uint32_t rank, uint32_t gridW, uint32_t* x, uint32_t* y) {
+    const uint32_t tilesX = gridW / kSensorTile;
+    const uint32_t tile = rank >> 6, ty = tile / tilesX, tx = tile - ty * tilesX;
+    *x = tx * kSensorTile + ((rank & 1) | ((rank >> 1) & 2) | ((rank >> 2) & 4));
+    *y = ty * kSensorTile + (((rank >> 1) & 1) | ((rank >> 2) & 2) | ((rank >> 3) & 4));
+}
+__device__ __forceinline__ uint32_t tileRank(uint32_t x, uint32_t y, uint32_t gridW) {
+    const uint32_t tile = (y / kSensorTile) * (gridW / kSensorTile) + x / kSensorTile;
+    const uint32_t in = (x & 1) | ((y & 1) << 1) | ((x & 2) << 1) | ((y & 2) << 2) | ((x & 4) << 2) | ((y & 4) << 3);
+    return tile * (kSensorTile * kSensorTile) + in;
+}
+static_assert(kSensorTile == 8, "three bits per axis inside a tile");
+
 // ---------------------------------------------------------------------------
 // Camera
 // ---------------------------------------------------------------------------

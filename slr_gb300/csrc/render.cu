@@ -104,16 +104,6 @@ __device__ __forceinline__ void tellHost(const WaveState &ws, const uint32_t* ro
     __threadfence_system();
 }
 
-// The reference's renderers sample the sensor in whole 8x8 tiles
-// (ImageSensor.cpp:13-14, :42-43; PTRenderer.cpp:104-110), also where a tile
-// hangs over the image's right or bottom edge; ImageSensor::add
-// (ImageSensor.cpp:125-130) clamps those samples into the last column / row.
-// A wave therefore traces every position of the tile-padded sample grid.
-constexpr uint32_t kSensorTile = 8;
-__host__ __device__ __forceinline__ uint32_t padToTile(uint32_t n) {
-    return (n + kSensorTile - 1) / kSensorTile * kSensorTile;
-}
-
 // Image sizes every entry point accepts: both sides positive and at most
 // 2^20 (so the tile padding cannot wrap a 32-bit side), and at most 2^31 - 1
 // positions in the tile-padded grid (path and film indices are 32-bit).
@@ -174,18 +164,12 @@ struct WaveParams {
 __device__ __forceinline__ void pathPosition(const WaveSegment &sg, uint32_t q, uint32_t* s, uint32_t* x, uint32_t* y) {
     const uint32_t rank = q / sg.samples;
     *s = q - rank * sg.samples;
-    const uint32_t tilesX = sg.gridW / kSensorTile;
-    const uint32_t tile = rank >> 6, ty = tile / tilesX, tx = tile - ty * tilesX;
-    *x = tx * kSensorTile + ((rank & 1) | ((rank >> 1) & 2) | ((rank >> 2) & 4));
-    *y = ty * kSensorTile + (((rank >> 1) & 1) | ((rank >> 2) & 2) | ((rank >> 3) & 4));
+    tilePosition(rank, sg.gridW, x, y);
 }
 // The first of the paths of grid position (x, y): its samples follow it.
 __device__ __forceinline__ uint32_t positionPath(const WaveSegment &sg, uint32_t x, uint32_t y) {
-    const uint32_t tile = (y / kSensorTile) * (sg.gridW / kSensorTile) + x / kSensorTile;
-    const uint32_t in = (x & 1) | ((y & 1) << 1) | ((x & 2) << 1) | ((y & 2) << 2) | ((x & 4) << 2) | ((y & 4) << 3);
-    return sg.pathBegin + (tile * (kSensorTile * kSensorTile) + in) * sg.samples;
+    return sg.pathBegin + tileRank(x, y, sg.gridW) * sg.samples;
 }
-static_assert(kSensorTile == 8, "three bits per axis inside a tile");
 
 // Per-bounce counter block: [0, kNumClassQueues - 1) paths per shading
 // class, kCtrExt paths in the extension queue of the bounce, kCtrShadow
@@ -2446,9 +2430,6 @@ int RenderEngine::render(const DeviceScene &ds, const slrgpu_settings &s, float*
         CUDA_TRY(cudaMemcpyAsync(filmSum, filmState, planeBytes, cudaMemcpyHostToDevice, stream));
         CUDA_TRY(cudaMemcpyAsync(filmComp, filmState + (size_t)P * kNumLambda, planeBytes, cudaMemcpyHostToDevice,
                                  stream));
-    } else if (bidir) {
-        CUDA_TRY(cudaMemsetAsync(filmSum, 0, planeBytes, stream));
-        CUDA_TRY(cudaMemsetAsync(filmComp, 0, planeBytes, stream));
     }
     if (!bidir) CUDA_TRY(cudaMemsetAsync(ws->stats, 0, 4 * sizeof(unsigned long long), stream));
     // the render's start and end events, destroyed on every return path
@@ -2472,10 +2453,8 @@ int RenderEngine::render(const DeviceScene &ds, const slrgpu_settings &s, float*
     std::memset(&bst, 0, sizeof(bst));
     float* dst = filmOnDevice && film ? film : filmOut;
     if (bidir) {
-        rc = renderBpt(*bpt, ds, s, filmSum, filmComp, stream, &launches, profile ? &eventPool : nullptr, &bst);
+        rc = renderBpt(*bpt, ds, s, filmSum, filmComp, dst, stream, &launches, profile ? &eventPool : nullptr, &bst);
         if (rc != SLRGPU_OK) return rc;
-        kFilmToPixelMajor<<<waveGrids(256).accumulate, 256, 0, stream>>>(filmSum, dst, P);
-        ++launches;
     } else {
         rc = runWaves(ds, s, pl, *ws, filmSum, filmComp, dst, filmState != nullptr, filmState != nullptr, stream, lm,
                       &launches, rngTape, &bounceCounts);

@@ -80,13 +80,14 @@ struct RenderEngine {
     ~RenderEngine();
 };
 
-// Bidirectional path tracing (BPTRenderer) into a compensated 16-bin film
-// ([16][width * height] sum and compensation planes on the device, added
-// to).  eventPool non-null: per-kernel timing into stats->kernel_ms.
+// Bidirectional path tracing (BPTRenderer) into a pixel-major 16-bin film on
+// the device; filmSum and filmComp ([16][width * height]) carry the
+// compensated sums from wave to wave.  eventPool non-null: per-kernel timing
+// into stats->kernel_ms.
 BptEngine* bptEngineCreate();
 void bptEngineDestroy(BptEngine* e);
 int renderBpt(BptEngine &eng, const DeviceScene &ds, const slrgpu_settings &s, float* filmSum, float* filmComp,
-              cudaStream_t stream, uint64_t* launches, std::vector<cudaEvent_t>* eventPool,
+              float* film, cudaStream_t stream, uint64_t* launches, std::vector<cudaEvent_t>* eventPool,
               slrgpu_render_stats* stats);
 
 // Wave slots (serving): path state for up to `paths` paths in flight.
