@@ -495,6 +495,24 @@ __device__ __forceinline__ float vertexCos(const BptGeom &g, uint32_t flags, V3 
     return ((flags >> kVfKindShift) & 3u) == kVtxMedium ? 1.0f : absDot(d, xyz(g.ng));
 }
 
+// The Russian roulette probability min(importance(f x cos / pdf), 1) of
+// extending a subpath (BPTRenderer.cpp:215-262).  The importance is linear in
+// the spectrum, so the density divides it once, behind one rounding
+// instead of sixteen; a zero density divides each wavelength as the reference
+// does (0 / 0 in one of them makes the weight invalid).  A connection takes
+// four of these: 64 divisions less brought the connections of the 512 x 512 x 4
+// box from 2.54 to 1.88 ms.
+__device__ __forceinline__ float extendRR(const Spec &f, float cosTerm, float pdf, int sel) {
+    Spec t;
+#pragma unroll
+    for (int q = 0; q < kNumLambda; ++q) t.v[q] = f.v[q] * cosTerm;
+    if (pdf != 0.0f) return stdMin(importance(t, sel) / pdf, 1.0f);
+#pragma unroll 1
+    for (int q = 0; q < kNumLambda; ++q)
+        if (f.v[q] * cosTerm == 0.0f) return __int_as_float(0x7fc00000);
+    return 1.0f;
+}
+
 // Closest hits of the bounce's subpaths, with the dynamic ray fetch of the path
 // tracer's extension kernel.  Apart from the bounce kernel, whose 128
 // registers leave 16 warps an SM, the walks have 32 to hide their node fetches.
@@ -754,10 +772,7 @@ __global__ void __launch_bounds__(256, 2) kBptBounce(DevScene sc, BptState st, c
                             // reverse densities of the previous vertex
                             BptPdf* prev = &st.pdf[(size_t)(k - 1) * st.S + sp];
                             prev->revAreaPdf = revPdf * cosLast / dist2;
-                            Spec rv;
-#pragma unroll
-                            for (int c = 0; c < kNumLambda; ++c) rv.v[c] = revFs.v[c] * cosOut / revPdf;
-                            prev->revRRProb = stdMin(importance(rv, sel), 1.0f);
+                            prev->revRRProb = extendRR(revFs, cosOut, revPdf, sel);
                             storeAlpha(st.alphaPend, sp, alpha);
                             st.rayOrg[sp] = make_float4(P.x, P.y, P.z, kRayEpsilon);
                             st.rayDir[sp] = make_float4(vecIn.x, vecIn.y, vecIn.z, 0.0f);
@@ -790,24 +805,6 @@ __device__ __forceinline__ void vertexBsdf(const DevScene &sc, const BptState &s
     } else {
         makeBsdf(sc, sc.materials[material], lambdas, (flags & kVfWlSelected) != 0, B);
     }
-}
-
-// The Russian roulette probability min(importance(f x cos / pdf), 1) of
-// extending a subpath (BPTRenderer.cpp:215-262).  The importance is linear in
-// the spectrum, so the density divides it once, behind one rounding
-// instead of sixteen; a zero density divides each wavelength as the reference
-// does (0 / 0 in one of them makes the weight invalid).  A connection takes
-// four of these: 64 divisions less brought the connections of the 512 x 512 x 4
-// box from 2.54 to 1.88 ms.
-__device__ __forceinline__ float extendRR(const Spec &f, float cosTerm, float pdf, int sel) {
-    Spec t;
-#pragma unroll
-    for (int q = 0; q < kNumLambda; ++q) t.v[q] = f.v[q] * cosTerm;
-    if (pdf != 0.0f) return stdMin(importance(t, sel) / pdf, 1.0f);
-#pragma unroll 1
-    for (int q = 0; q < kNumLambda; ++q)
-        if (f.v[q] * cosTerm == 0.0f) return __int_as_float(0x7fc00000);
-    return 1.0f;
 }
 
 // One connection (BPTRenderer.cpp:174-280; VOL: VolumetricBPTRenderer.cpp:
