@@ -1402,48 +1402,101 @@ __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kShadowVolMediu
 // lanes per pixel, each with four wavelengths and film bins: a sample's 64
 // bytes of radiance are one access of the quad, and a pixel's samples, which
 // lie next to each other, stream, four of them loaded ahead of the sums'
-// chain.  One thread per pixel took 0.42 ms on a 333 x 187 image with 24
-// samples, whose last pixel alone sums 576 (this kernel 0.23 ms), and sixteen
-// lanes repeated the per-sample work too often (1024 x 1024 x 64: 4.4 ms
-// against 1.8 ms, 3.5 TB/s; eight samples loaded ahead at 115 registers 2.3).
+// chain.  One thread per pixel had too few chains in flight on small images;
+// sixteen lanes repeated the per-sample work too often (1024 x 1024 x 64: 4.4
+// ms against 1.7 ms, 3.9 TB/s; eight samples loaded ahead at 115 registers
+// 2.3).
 // A render's first wave starts from zero sums without reading them, and its
 // last one writes the pixel-major film itself.
 constexpr uint32_t kFilmFirst = 1u;   // the film's sums start at zero: do not read them
 constexpr uint32_t kFilmKeep = 2u;    // store sums and compensations for a later wave
+constexpr uint32_t kFilmLanes = 4, kFilmBins = kNumLambda / kFilmLanes;
+
+// What a path adds to the four bins of a quad's lane; false for a dropped
+// (non-finite) sample.  Called by the four lanes of `quad`.
+__device__ __forceinline__ bool filmAddend(float4 Lv, float w, float wlOff, uint32_t bin0, uint32_t quad,
+                                           float addend[kFilmBins]) {
+    const float recBinWidth = kNumLambda / (kWavelengthHigh - kWavelengthLow);
+    const float c[kFilmBins] = {Lv.x * w, Lv.y * w, Lv.z * w, Lv.w * w};
+    // Wavelength i of a path falls in film bin i unless rounding moves it
+    // across a bin edge; then every bin sums its wavelengths in order.  0 + x
+    // keeps the sign of zero the summing loop gives.
+    bool finite = true, own = true;
+    uint32_t bins[kFilmBins];
+#pragma unroll
+    for (uint32_t b = 0; b < kFilmBins; ++b) {
+        const float lam = lambdaAt((int)(bin0 + b), wlOff);
+        const float f = __fmul_rn(divRange(__fsub_rn(lam, kWavelengthLow)), (float)kNumLambda);
+        bins[b] = min((uint32_t)f, (uint32_t)(kNumLambda - 1));
+        own &= bins[b] == bin0 + b;
+        finite &= isfinite(c[b]);
+        addend[b] = __fadd_rn(0.0f, __fmul_rn(c[b], recBinWidth));
+    }
+    if (__ballot_sync(quad, finite && own) != quad) {
+        if (__ballot_sync(quad, finite) != quad) return false;
+#pragma unroll
+        for (uint32_t b = 0; b < kFilmBins; ++b) addend[b] = 0.0f;
+#pragma unroll
+        for (uint32_t i = 0; i < kNumLambda; ++i) {
+            const uint32_t bi = __shfl_sync(quad, bins[i % kFilmBins], i / kFilmBins, kFilmLanes);
+            const float ci = __shfl_sync(quad, c[i % kFilmBins], i / kFilmBins, kFilmLanes);
+#pragma unroll
+            for (uint32_t b = 0; b < kFilmBins; ++b)
+                if (bi == bin0 + b) addend[b] = __fmaf_rn(ci, recBinWidth, addend[b]);
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ void filmAdd(float sum[kFilmBins], float comp[kFilmBins], const float addend[kFilmBins]) {
+#pragma unroll
+    for (uint32_t b = 0; b < kFilmBins; ++b) {
+        const float cin = __fsub_rn(addend[b], comp[b]);
+        const float st = __fadd_rn(sum[b], cin);
+        comp[b] = __fsub_rn(__fsub_rn(st, sum[b]), cin);
+        sum[b] = st;
+    }
+}
+__device__ __forceinline__ void filmLoad(const WaveSegment &sg, uint32_t pix, uint32_t bin0, uint32_t flags,
+                                         float sum[kFilmBins], float comp[kFilmBins]) {
+#pragma unroll
+    for (uint32_t b = 0; b < kFilmBins; ++b) {
+        const size_t at = (size_t)(bin0 + b) * (sg.width * sg.height) + pix;
+        sum[b] = flags & kFilmFirst ? 0.0f : sg.filmSum[at];
+        comp[b] = flags & kFilmFirst ? 0.0f : sg.filmComp[at];
+    }
+}
+__device__ __forceinline__ void filmStore(const WaveSegment &sg, uint32_t pix, uint32_t bin0, uint32_t flags,
+                                          const float sum[kFilmBins], const float comp[kFilmBins], float* out) {
+#pragma unroll
+    for (uint32_t b = 0; b < kFilmBins; ++b) {
+        const size_t at = (size_t)(bin0 + b) * (sg.width * sg.height) + pix;
+        if (flags & kFilmKeep) {
+            sg.filmSum[at] = sum[b];
+            sg.filmComp[at] = comp[b];
+        }
+        if (out) out[(size_t)pix * kNumLambda + bin0 + b] = sum[b];
+    }
+}
+
 __global__ void __launch_bounds__(256, 3) kAccumulate(WaveState ws, const __grid_constant__ WaveParams wpArg,
-                                                   const WaveParams* __restrict__ wpDev, uint32_t flags, float* out) {
+                                                      const WaveParams* __restrict__ wpDev, uint32_t flags, float* out) {
     waveBegin(false);
     const WaveParams &wp = wpDev ? *wpDev : wpArg;
-    const float recBinWidth = kNumLambda / (kWavelengthHigh - kWavelengthLow);
-    constexpr uint32_t kLanes = 4, kBins = kNumLambda / kLanes;
-    const uint32_t lane = threadIdx.x & (kLanes - 1), bin0 = lane * kBins;
+    const uint32_t lane = threadIdx.x & (kFilmLanes - 1), bin0 = lane * kFilmBins;
     const uint32_t quad = 0xfu << (threadIdx.x & 28);
-    const uint32_t step = gridDim.x * blockDim.x / kLanes;
+    const uint32_t threads = gridDim.x * blockDim.x, thread = blockIdx.x * blockDim.x + threadIdx.x;
     const float4* L4 = reinterpret_cast<const float4*>(ws.L);
-    for (uint32_t fp = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes; fp < wp.filmPixels; fp += step) {
+    for (uint32_t fp = thread / kFilmLanes; fp < wp.filmPixels; fp += threads / kFilmLanes) {
         uint32_t k = 0;
         while (k + 1 < wp.numSegments && fp >= wp.seg[k + 1].filmBegin) ++k;
         const WaveSegment sg = wp.seg[k];
-        const uint32_t P = sg.width * sg.height;
         const uint32_t pix = fp - sg.filmBegin;
-        float sum[kBins], comp[kBins];
-#pragma unroll
-        for (uint32_t b = 0; b < kBins; ++b) {
-            const size_t at = (size_t)(bin0 + b) * P + pix;
-            sum[b] = comp[b] = 0.0f;
-            if (!(flags & kFilmFirst)) {
-                sum[b] = sg.filmSum[at];
-                comp[b] = sg.filmComp[at];
-            }
-        }
-        unsigned long long dropped = 0;
-        // Grid positions clamped into this pixel: itself, plus the overhang
-        // of the last column / row; samples in the order sample, row, column.
         const uint32_t x = pix % sg.width, y = pix / sg.width;
-        const uint32_t xEnd = x + 1 == sg.width ? sg.gridW : x + 1;
-        const uint32_t yEnd = y + 1 == sg.height ? sg.gridH : y + 1;
-        const uint32_t n = sg.samples * (xEnd - x) * (yEnd - y);
-        uint32_t s = 0, gx = x, gy = y;
+        if ((x + 1 == sg.width && sg.gridW > sg.width) || (y + 1 == sg.height && sg.gridH > sg.height)) continue;
+        float sum[kFilmBins], comp[kFilmBins];
+        filmLoad(sg, pix, bin0, flags, sum, comp);
+        unsigned long long dropped = 0;
+        const uint32_t first = positionPath(sg, x, y), n = sg.samples;
         constexpr uint32_t kAhead = 4;
         for (uint32_t i0 = 0; i0 < n; i0 += kAhead) {
             float4 Lv[kAhead];
@@ -1453,77 +1506,73 @@ __global__ void __launch_bounds__(256, 3) kAccumulate(WaveState ws, const __grid
                 Lv[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 w[j] = off[j] = 0.0f;
                 if (i0 + j < n) {
-                    const uint32_t p = positionPath(sg, gx, gy) + s;
-                    Lv[j] = L4[(size_t)p * kLanes + lane];
+                    const uint32_t p = first + i0 + j;
+                    Lv[j] = L4[(size_t)p * kFilmLanes + lane];
                     w[j] = ws.ps[p].camWeight;
                     off[j] = ws.ps[p].wlOffset;
-                    if (++gx == xEnd) {
-                        gx = x;
-                        if (++gy == yEnd) {
-                            gy = y;
-                            ++s;
-                        }
-                    }
                 }
             }
 #pragma unroll
             for (uint32_t j = 0; j < kAhead; ++j) {
                 if (i0 + j >= n) break;
-                const float c[kBins] = {Lv[j].x * w[j], Lv[j].y * w[j], Lv[j].z * w[j], Lv[j].w * w[j]};
-                // Wavelength i of a path falls in film bin i unless rounding
-                // moves it across a bin edge; then every bin sums its
-                // wavelengths in order.  0 + x keeps the sign of zero the
-                // summing loop gives.
-                bool finite = true, own = true;
-                uint32_t bins[kBins];
-#pragma unroll
-                for (uint32_t b = 0; b < kBins; ++b) {
-                    const float lam = lambdaAt((int)(bin0 + b), off[j]);
-                    const float f = __fmul_rn(divRange(__fsub_rn(lam, kWavelengthLow)), (float)kNumLambda);
-                    bins[b] = min((uint32_t)f, (uint32_t)(kNumLambda - 1));
-                    own &= bins[b] == bin0 + b;
-                    finite &= isfinite(c[b]);
-                }
-                float addend[kBins];
-#pragma unroll
-                for (uint32_t b = 0; b < kBins; ++b) addend[b] = __fadd_rn(0.0f, __fmul_rn(c[b], recBinWidth));
-                if (__ballot_sync(quad, finite && own) != quad) {
-                    if (__ballot_sync(quad, finite) != quad) {
-                        ++dropped;
-                        continue;
-                    }
-#pragma unroll
-                    for (uint32_t b = 0; b < kBins; ++b) addend[b] = 0.0f;
-#pragma unroll
-                    for (uint32_t i = 0; i < kNumLambda; ++i) {
-                        const uint32_t bi = __shfl_sync(quad, bins[i % kBins], i / kBins, kLanes);
-                        const float ci = __shfl_sync(quad, c[i % kBins], i / kBins, kLanes);
-#pragma unroll
-                        for (uint32_t b = 0; b < kBins; ++b)
-                            if (bi == bin0 + b) addend[b] = __fmaf_rn(ci, recBinWidth, addend[b]);
-                    }
-                }
-#pragma unroll
-                for (uint32_t b = 0; b < kBins; ++b) {
-                    const float cin = __fsub_rn(addend[b], comp[b]);
-                    const float st = __fadd_rn(sum[b], cin);
-                    comp[b] = __fsub_rn(__fsub_rn(st, sum[b]), cin);
-                    sum[b] = st;
-                }
+                float addend[kFilmBins];
+                if (filmAddend(Lv[j], w[j], off[j], bin0, quad, addend)) filmAdd(sum, comp, addend);
+                else ++dropped;
             }
         }
-#pragma unroll
-        for (uint32_t b = 0; b < kBins; ++b) {
-            const size_t at = (size_t)(bin0 + b) * P + pix;
-            if (flags & kFilmKeep) {
-                sg.filmSum[at] = sum[b];
-                sg.filmComp[at] = comp[b];
-            }
-            if (out) out[(size_t)pix * kNumLambda + bin0 + b] = sum[b];
-        }
+        filmStore(sg, pix, bin0, flags, sum, comp, out);
         if (dropped && lane == 0) {
             atomicAdd(&ws.stats[2], dropped);
             if (sg.dropped) atomicAdd(sg.dropped, dropped);
+        }
+    }
+    // The last column and row of an image that ends inside a sensor tile take
+    // the overhang's grid positions too, up to 64 for one pixel, and their
+    // sums are one chain each: a warp per pixel, whose eight quads prepare
+    // eight samples at once (order: sample, row, column).  333 x 187 x 24, 576
+    // samples in the corner: 0.23 ms with a quad per pixel, 0.15 so.
+    const uint32_t warpLane = threadIdx.x & 31;
+    for (uint32_t k = 0; k < wp.numSegments; ++k) {
+        if (wp.seg[k].gridW == wp.seg[k].width && wp.seg[k].gridH == wp.seg[k].height) continue;
+        const WaveSegment sg = wp.seg[k];
+        const uint32_t column = sg.gridW > sg.width ? sg.height : 0;
+        const uint32_t edge = column + (sg.gridH > sg.height ? sg.width - (column ? 1 : 0) : 0);
+        for (uint32_t e = thread >> 5; e < edge; e += threads >> 5) {
+            const uint32_t x = e < column ? sg.width - 1 : e - column, y = e < column ? e : sg.height - 1;
+            const uint32_t pix = y * sg.width + x;
+            const uint32_t nx = x + 1 == sg.width ? sg.gridW - x : 1, ny = y + 1 == sg.height ? sg.gridH - y : 1;
+            const uint32_t n = sg.samples * nx * ny;
+            float sum[kFilmBins], comp[kFilmBins];
+            filmLoad(sg, pix, bin0, flags, sum, comp);
+            unsigned long long dropped = 0;
+            for (uint32_t i0 = 0; i0 < n; i0 += 8) {
+                const uint32_t i = i0 + warpLane / kFilmLanes;
+                float4 Lv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                float w = 0.0f, off = 0.0f, addend[kFilmBins];
+                if (i < n) {
+                    const uint32_t s = i / (nx * ny), g = i - s * (nx * ny), gy = g / nx;
+                    const uint32_t p = positionPath(sg, x + (g - gy * nx), y + gy) + s;
+                    Lv = L4[(size_t)p * kFilmLanes + lane];
+                    w = ws.ps[p].camWeight;
+                    off = ws.ps[p].wlOffset;
+                }
+                const uint32_t ok = __ballot_sync(0xffffffffu, filmAddend(Lv, w, off, bin0, quad, addend));
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) {
+                    float a[kFilmBins];
+#pragma unroll
+                    for (uint32_t b = 0; b < kFilmBins; ++b)
+                        a[b] = __shfl_sync(0xffffffffu, addend[b], j * kFilmLanes + lane);
+                    if (i0 + j >= n) continue;
+                    if ((ok >> (j * kFilmLanes)) & 1u) filmAdd(sum, comp, a);
+                    else ++dropped;
+                }
+            }
+            if (warpLane < kFilmLanes) filmStore(sg, pix, bin0, flags, sum, comp, out);
+            if (dropped && warpLane == 0) {
+                atomicAdd(&ws.stats[2], dropped);
+                if (sg.dropped) atomicAdd(sg.dropped, dropped);
+            }
         }
     }
 }
