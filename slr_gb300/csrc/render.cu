@@ -290,9 +290,16 @@ __global__ void kRaygen(DevScene scArg, WaveState ws, const __grid_constant__ Wa
 #ifndef SLRGPU_TRACE_REFILL
 #define SLRGPU_TRACE_REFILL 1
 #endif
-// The same threshold for the ray-query kernel (slrgpu_trace_rays).
+// The same two for the ray-query kernel (slrgpu_trace_rays), whose refill costs a
+// shared-memory atomic only: looks every 16, 8 and 6 visits took 401, 380 and 377
+// us for 1,000,003 incoherent closest-hit queries on 24k triangles, 1469, 1448
+// and 1427 us for 4 Mi any-hit queries on 176k, and 398, 403 and 405 us for 2 Mi
+// coherent ones.
 #ifndef SLRGPU_QUERY_REFILL_LANES
 #define SLRGPU_QUERY_REFILL_LANES SLRGPU_TRACE_REFILL_LANES
+#endif
+#ifndef SLRGPU_QUERY_REFILL_VISITS
+#define SLRGPU_QUERY_REFILL_VISITS 6
 #endif
 static_assert(SLRGPU_QUERY_REFILL_LANES >= 1 && SLRGPU_QUERY_REFILL_LANES <= 32, "a warp has 32 lanes");
 
@@ -1605,6 +1612,8 @@ __device__ __forceinline__ void traceQueries(const DevScene &sc, const float4* _
     __syncthreads();
     const uint32_t width = (uint32_t)min((chunk + 7) / 8, (uint64_t)32);
     const uint32_t refill = min(width, (uint32_t)SLRGPU_QUERY_REFILL_LANES);
+    // a block whose rays all start at once has none to look for
+    const int visits = chunk > blockDim.x ? SLRGPU_QUERY_REFILL_VISITS : 1 << 20;
     ClosestStack cstack(shared);
     LocalStack<uint32_t> astack;
     ClosestWalk<WT> cw;
@@ -1632,8 +1641,7 @@ __device__ __forceinline__ void traceQueries(const DevScene &sc, const float4* _
             }
         }
         if (live && !fin)
-            fin = ANY ? aw.advance(sc, astack, SLRGPU_TRACE_REFILL_VISITS)
-                      : cw.advance(sc, cstack, SLRGPU_TRACE_REFILL_VISITS);
+            fin = ANY ? aw.advance(sc, astack, visits) : cw.advance(sc, cstack, visits);
         if (live && fin) {
             if (ANY) {
                 prim[i] = aw.occluded ? 1u : 0u;

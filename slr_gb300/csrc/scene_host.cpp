@@ -1015,6 +1015,7 @@ struct WideBuilder {
             f.prim = prim;
             f.e1x = p[3] - p[0]; f.e1y = p[4] - p[1]; f.e1z = p[5] - p[2]; f.pad0 = 0;
             f.e2x = p[6] - p[0]; f.e2y = p[7] - p[1]; f.e2z = p[8] - p[2]; f.pad1 = 0;
+            f.pad2[0] = f.pad2[1] = f.pad2[2] = f.pad2[3] = 0;
             out->frags.push_back(f);
         }
         return kLeafBit | ((count - 1) << kLeafCountShift) | first;

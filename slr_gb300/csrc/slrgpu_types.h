@@ -90,13 +90,14 @@ struct alignas(128) BvhNode {
 };
 static_assert(sizeof(BvhNode) == 32 * kBvhWidth, "whole cache lines");
 
-// Traversal fragment (48 B, leaf order): v0.xyz + prim id bits, e01 = p1 - p0,
+// Traversal fragment (64 B, two whole sectors, leaf order): v0.xyz + prim id bits, e01 = p1 - p0,
 // e02 = p2 - p0 (precomputed with the same float subtraction as the test).
-struct TriFrag {
+struct alignas(32) TriFrag {
     float v0x, v0y, v0z;
     uint32_t prim;
     float e1x, e1y, e1z, pad0;
     float e2x, e2y, e2z, pad1;
+    float pad2[4];
 };
 
 struct DevCamera {
