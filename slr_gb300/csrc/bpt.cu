@@ -499,7 +499,8 @@ __device__ __forceinline__ float vertexCos(const BptGeom &g, uint32_t flags, V3 
 // extending a subpath (BPTRenderer.cpp:215-262).  The importance is linear in
 // the spectrum, so the density divides it once, behind one rounding
 // instead of sixteen; a zero density divides each wavelength as the reference
-// does (0 / 0 in one of them makes the weight invalid).  A connection takes
+// does (0 / 0 in one of them, or a NaN of vertices that lie in one plane, makes
+// the weight invalid).  A connection takes
 // four of these: 64 divisions less brought the connections of the 512 x 512 x 4
 // box from 2.54 to 1.88 ms.
 __device__ __forceinline__ float extendRR(const Spec &f, float cosTerm, float pdf, int sel) {
@@ -509,7 +510,7 @@ __device__ __forceinline__ float extendRR(const Spec &f, float cosTerm, float pd
     if (pdf != 0.0f) return stdMin(importance(t, sel) / pdf, 1.0f);
 #pragma unroll 1
     for (int q = 0; q < kNumLambda; ++q)
-        if (f.v[q] * cosTerm == 0.0f) return __int_as_float(0x7fc00000);
+        if (!(fabsf(f.v[q] * cosTerm) > 0.0f)) return __int_as_float(0x7fc00000);
     return 1.0f;
 }
 

@@ -2004,7 +2004,11 @@ cudaError_t BounceCounts::get(uint32_t bounce, cudaStream_t stream, uint32_t* co
         if ((spins & 0xfff) == 0) {
             // a stream that has run dry has written the word, or failed
             const cudaError_t e = cudaStreamQuery(stream);
-            if (e == cudaErrorNotReady) continue;
+            if (e == cudaErrorNotReady) {
+                // not an error: leave no trace for the check after the wave
+                if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();
+                continue;
+            }
             v = *word;
             *count = (uint32_t)v;
             return e != cudaSuccess ? e : ((uint32_t)(v >> 32) == tag ? cudaSuccess : cudaErrorUnknown);
