@@ -84,13 +84,13 @@ BYTES_BPT_SHADOW = 164   # queued connection 100 B in, any-hit query, 64 B atomi
 # units of those launches (slrgpu_context_queue_counts of the same frame).
 # The line scales them by the units per launch of the measured workload (the
 # full-size run is not captured with more than the launch list).
-# kExtendSort, bounces 0-2: 171.8 MB over 1,604,943 closest-hit queries (the
+# kExtendSort, bounces 0-2: 159.4 MB over 1,604,943 closest-hit queries (the
 # BVH nodes and triangles that miss L2, the path records of the roulette at
 # the hit, the hit records).
-EXTEND_DRAM_BYTES_PER_UNIT = 107.0
-# kShadeSurf, the first three launches (bounce 0 conductor and dielectric,
-# bounce 1 conductor): 258.8 MB over 610,018 shaded paths.
-SHADE_DRAM_BYTES_PER_UNIT = 424.3
+EXTEND_DRAM_BYTES_PER_UNIT = 99.3
+# kShadeSurf, bounce 0 conductor and dielectric and bounce 1 conductor: 166.8
+# MB over 610,018 shaded paths.
+SHADE_DRAM_BYTES_PER_UNIT = 273.5
 
 
 def load_peaks():
