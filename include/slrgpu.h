@@ -99,7 +99,8 @@ typedef struct slrgpu_settings {
  * allocation-free render and the server return SLRGPU_ERR_UNSUPPORTED. */
 #define SLRGPU_FLAG_BPT 4u
 
-/* Kernel classes of the wavefront (index into kernel_ms / kernel_count). */
+/* Kernel classes of the wavefront (index into kernel_ms / kernel_count); the
+ * kernel that takes a bounce of few paths to its end counts as shading. */
 #define SLRGPU_KERNEL_RAYGEN 0
 #define SLRGPU_KERNEL_EXTEND 1
 #define SLRGPU_KERNEL_SHADE 2
