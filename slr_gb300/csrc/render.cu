@@ -50,7 +50,7 @@ struct __align__(16) PathScalars {
 };
 static_assert(sizeof(PathScalars) == 32, "one sector per path");
 
-constexpr int kCtrStride = 14;   // words of a bounce's counter block, see kCtr*
+constexpr int kCtrStride = 17;   // words of a bounce's counter block, see kCtr*
 
 struct WaveState {
     float4* ray;         // [N][2]: origin xyz + tmin, direction xyz + tmax (one sector per path)
@@ -87,14 +87,48 @@ struct WaveState {
 // latencies and not the sum (64 x 64 x 1 box: 526 to 392 us, the 176k-triangle
 // terrain at 512 x 512 x 4: 3.33 to 2.35 ms, every kind of BSDF at 333 x 187 x
 // 24: 3.36 to 2.17 ms).
+//
+// What a beside kernel reads was written by grids that its predecessor waited
+// for, and only that wait (griddepcontrol.wait) makes their writes visible: the
+// predecessor's trigger does not, and the kernel has not waited itself.  So the
+// "after" kernel at the head of such a chain hands the visibility on: once its
+// wait is over it stores its mark with release semantics, and every block of
+// the kernels beside it loads the mark with acquire semantics before its first
+// read of the path state.  The mark is stored before the trigger, so a block
+// finds it set; one that does not has the other documented way, the wait
+// for its predecessor.  Marks are words of the bounce's counter block, zero
+// when the wave starts.  Counts and queues are never read through the
+// read-only path (const __restrict__): they change while a waiting kernel is
+// already resident.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void waveBegin(bool beside) {
-    if (!beside) asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+__device__ __forceinline__ void waveWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void waveTrigger() {
+    if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// The start of an "after" kernel; mark: for the kernels beside it, or null.
+__device__ __forceinline__ void waveBeginAfter(uint32_t* mark) {
+    waveWait();
+    if (mark && blockIdx.x == 0 && threadIdx.x == 0)
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(mark), "r"(1u) : "memory");
+    waveTrigger();
+}
+// The start of a kernel beside the one that stores `mark`, or beside another such.
+__device__ __forceinline__ void waveBeginBeside(const uint32_t* mark) {
+    uint32_t seen = 1;
+    if (threadIdx.x == 0) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(mark) : "memory");
+    if (!__syncthreads_and((int)seen)) waveWait();
+    waveTrigger();
 }
 // One thread holds the kernel's completion for the predecessor's.
+__device__ __forceinline__ void waveEndBeside() {
+    if (blockIdx.x == 0 && threadIdx.x == 0) asm volatile("griddepcontrol.wait;");
+}
+__device__ __forceinline__ void waveBegin(uint32_t* mark, bool beside) {
+    if (beside) waveBeginBeside(mark);
+    else waveBeginAfter(mark);
+}
 __device__ __forceinline__ void waveEnd(bool beside) {
-    if (beside && blockIdx.x == 0 && threadIdx.x == 0) asm volatile("griddepcontrol.wait;");
+    if (beside) waveEndBeside();
 }
 // The host's view of a bounce's size, written as the bounce starts.
 __device__ __forceinline__ void tellHost(const WaveState &ws, const uint32_t* rowCounters, uint32_t n) {
@@ -188,6 +222,9 @@ constexpr int kCtrMedShadow = 9;
 constexpr int kCtrMedTake = 10;
 constexpr int kCtrExtTake = 11;
 constexpr int kCtrShadowTake = 12;
+constexpr int kCtrExtMark = 14;       // marks of the launch order: the extension kernel's,
+constexpr int kCtrVolMark = 15;       // the medium collision kernel's,
+constexpr int kCtrShadeMark = 16;     // and the first shading kernel's
 constexpr int kCtrTailRow = 13;       // row 0 only: 1 + the bounce that kTail starts at, 0 while there is none
 // hit.w of a path whose ray stopped at a collision in the medium (hit.x = its
 // distance, hit.y = 1 inside the density grid's unit cube)
@@ -225,7 +262,7 @@ __global__ void kRaygen(DevScene scArg, WaveState ws, const __grid_constant__ Wa
                         const WaveParams* __restrict__ wpDev, const DevScene* __restrict__ scenes,
                         bool initAlpha, uint32_t tailPaths) {
     const WaveParams &wp = wpDev ? *wpDev : wpArg;
-    waveBegin(false);
+    waveBeginAfter(nullptr);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         ws.counters[kCtrExt] = wp.numPaths;
         if (wp.numPaths <= tailPaths) ws.counters[kCtrTailRow] = 1;
@@ -309,7 +346,7 @@ static_assert(SLRGPU_QUERY_REFILL_LANES >= 1 && SLRGPU_QUERY_REFILL_LANES <= 32,
 // queue (medQueue) instead.
 template <bool MULTI, bool WT, bool VOL = false>
 __device__ __forceinline__ void shadowRefill(const DevScene &scArg, const WaveState &ws,
-                                             const uint32_t* __restrict__ queue, uint32_t n, uint32_t* cursor,
+                                             const uint32_t* queue, uint32_t n, uint32_t* cursor,
                                              const DevScene* __restrict__ scenes, uint32_t* medQueue = nullptr,
                                              uint32_t* medCount = nullptr) {
     LocalStack<uint32_t> stack;
@@ -347,11 +384,11 @@ __device__ __forceinline__ void shadowRefill(const DevScene &scArg, const WaveSt
 
 template <bool MULTI>
 __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadow(DevScene scArg, WaveState ws,
-                                                                      const uint32_t* __restrict__ queue,
-                                                                      const uint32_t* __restrict__ count,
-                                                                      uint32_t* cursor,
+                                                                      const uint32_t* queue,
+                                                                      const uint32_t* count,
+                                                                      uint32_t* cursor, const uint32_t* mark,
                                                                       const DevScene* __restrict__ scenes) {
-    waveBegin(true);
+    waveBeginBeside(mark);
     const uint32_t n = *count;
 #if SLRGPU_TRACE_REFILL
     if (n == 0) {
@@ -370,7 +407,7 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadow(DevScene
     }
 #endif
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ws.stats[1], (unsigned long long)n);
-    waveEnd(true);
+    waveEndBeside();
 }
 
 // ---------------------------------------------------------------------------
@@ -432,7 +469,7 @@ __device__ __forceinline__ void pushByClass(const WaveState &ws, uint32_t* class
 // SORT: push each path to the queue of its shading class.
 template <bool MULTI, bool WT, bool SORT = true>
 __device__ __forceinline__ void extendRefill(const DevScene &scArg, const WaveState &ws,
-                                             const uint32_t* __restrict__ queue, uint32_t n, uint32_t* cursor,
+                                             const uint32_t* queue, uint32_t n, uint32_t* cursor,
                                              uint32_t* classCounts, const DevScene* __restrict__ scenes,
                                              StackEntry* shared, uint32_t maxDepth = 0) {
     ClosestStack stack(shared);
@@ -465,11 +502,11 @@ __device__ __forceinline__ void extendRefill(const DevScene &scArg, const WaveSt
 
 template <bool MULTI>
 __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kExtendSort(DevScene scArg, WaveState ws,
-                                                                          const uint32_t* __restrict__ queue,
-                            const uint32_t* __restrict__ count, uint32_t* classCounts, uint32_t* cursor,
+                                                                          const uint32_t* queue,
+                            const uint32_t* count, uint32_t* classCounts, uint32_t* cursor,
                             uint32_t maxDepth, uint32_t tailPaths, const DevScene* __restrict__ scenes) {
     __shared__ StackEntry shared[kSharedStackEntries * 256];
-    waveBegin(false);
+    waveBeginAfter(classCounts + kCtrExtMark);
     const uint32_t n = *count;
     tellHost(ws, classCounts, n);
     if (n <= tailPaths) {   // kTail's (or no paths)
@@ -504,11 +541,10 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kExtendSort(DevS
 // Closest hits of the volumetric path tracer's extension rays (the medium
 // interaction comes after, in kVolInteract).
 __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kExtend(DevScene sc, WaveState ws,
-                                                                      const uint32_t* __restrict__ queue,
-                                                                      const uint32_t* __restrict__ count,
+                                                                      const uint32_t* queue, uint32_t* count,
                                                                       uint32_t* cursor) {
     __shared__ StackEntry shared[kSharedStackEntries * 256];
-    waveBegin(false);
+    waveBeginAfter(count + (kCtrExtMark - kCtrExt));
     const uint32_t n = *count;
     tellHost(ws, count, n);
     if (n == 0) return;
@@ -562,9 +598,10 @@ __device__ __forceinline__ void shadeMiss(const DevScene &scArg, const WaveState
 }
 
 template <bool MULTI>
-__global__ void kShadeMiss(DevScene scArg, WaveState ws, const uint32_t* __restrict__ queue,
-                           const uint32_t* __restrict__ count, const DevScene* __restrict__ scenes, bool beside) {
-    waveBegin(beside);
+__global__ void kShadeMiss(DevScene scArg, WaveState ws, const uint32_t* queue,
+                           const uint32_t* count, const DevScene* __restrict__ scenes, uint32_t* mark,
+                           bool beside) {
+    waveBegin(mark, beside);
     const uint32_t n = *count;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         shadeMiss<MULTI>(scArg, ws, queue[i], scenes);
@@ -826,11 +863,11 @@ __device__ __forceinline__ void shadeVertex(const DevScene &scArg, const WaveSta
 template <int K, bool MULTI>
 __global__ void __launch_bounds__(256, K == kMatGGXScattering ? SLRGPU_SHADE_DIELECTRIC_MIN_BLOCKS
                                                                : SLRGPU_SHADE_MIN_BLOCKS) kShadeSurf(DevScene scArg, WaveState ws, uint32_t maxDepth,
-                                                  const uint32_t* __restrict__ inQueue,
-                                                  const uint32_t* __restrict__ inCount, uint32_t* outQueue,
+                                                  const uint32_t* inQueue,
+                                                  const uint32_t* inCount, uint32_t* outQueue,
                                                   uint32_t* outCount, uint32_t* shQueue, uint32_t* shCount,
-                                                  const DevScene* __restrict__ scenes, bool beside) {
-    if (!MULTI) waveBegin(beside);   // waves of several scenes launch in plain order
+                                                  const DevScene* __restrict__ scenes, uint32_t* mark, bool beside) {
+    if (!MULTI) waveBegin(mark, beside);   // waves of several scenes launch in plain order
     const uint32_t n = *inCount;
     __shared__ float sAlpha[SLRGPU_SHADE_SMEM_ALPHA ? kNumLambda * 256 : 1];
     // the surface point likewise, from the BSDF query to the new ray
@@ -890,11 +927,11 @@ __global__ void __launch_bounds__(256, 1) kTail(DevScene scArg, WaveState ws, ui
                                                                    const DevScene* __restrict__ scenes) {
     __shared__ float sAlpha[SLRGPU_SHADE_SMEM_ALPHA ? kNumLambda * 256 : 1];
     __shared__ float sSurf[SLRGPU_SHADE_SMEM_SP ? 15 * 256 : 1];
-    waveBegin(false);
+    waveBeginAfter(nullptr);
     if (ws.counters[kCtrTailRow] == 0) return;
     const uint32_t b = ws.counters[kCtrTailRow] - 1;
     const uint32_t n = ws.counters[(size_t)kCtrStride * b + kCtrExt];
-    const uint32_t* __restrict__ queue = ws.queue[b & 1];
+    const uint32_t* queue = ws.queue[b & 1];
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     // warps of different SMs first: consecutive ranges go to consecutive blocks
@@ -993,10 +1030,10 @@ __global__ void __launch_bounds__(256, 1) kTail(DevScene scArg, WaveState ws, ui
 // interaction from the shading keeps each shading kernel's code to one
 // vertex kind.
 __global__ void __launch_bounds__(256, SLRGPU_VOLINTERACT_MIN_BLOCKS) kVolInteract(DevScene sc, WaveState ws,
-                                                                              const uint32_t* __restrict__ queue,
-                                                                              const uint32_t* __restrict__ count,
+                                                                              const uint32_t* queue,
+                                                                              const uint32_t* count,
                                                                               uint32_t* classCounts) {
-    waveBegin(false);
+    waveBeginAfter(classCounts + kCtrVolMark);
     const uint32_t n = *count;
     const float inf = __int_as_float(0x7f800000);
     const DevMedium &med = sc.medium;
@@ -1048,11 +1085,11 @@ __global__ void __launch_bounds__(256, SLRGPU_VOLINTERACT_MIN_BLOCKS) kVolIntera
 
 template <int K>
 __global__ void __launch_bounds__(256, SLRGPU_SHADEVOL_MIN_BLOCKS) kShadeVol(DevScene sc, WaveState ws, uint32_t maxDepth,
-                                                 const uint32_t* __restrict__ inQueue,
-                                                 const uint32_t* __restrict__ inCount, uint32_t* outQueue,
+                                                 const uint32_t* inQueue,
+                                                 const uint32_t* inCount, uint32_t* outQueue,
                                                  uint32_t* outCount, uint32_t* shQueue, uint32_t* shCount,
-                                                 bool beside) {
-    waveBegin(beside);
+                                                 uint32_t* mark, bool beside) {
+    waveBegin(mark, beside);
     const uint32_t n = *inCount;
     const float inf = __int_as_float(0x7f800000);
     const float twoPi = 6.28318530717958647692f;
@@ -1322,11 +1359,11 @@ __global__ void __launch_bounds__(256, SLRGPU_SHADEVOL_MIN_BLOCKS) kShadeVol(Dev
 // Scene.cpp:114-135): occlusion by surfaces here; unoccluded rays that may
 // cross the medium go to a second queue for their spectral transmittance.
 __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadowVol(DevScene sc, WaveState ws,
-                                                                         const uint32_t* __restrict__ queue,
-                                                                         const uint32_t* __restrict__ count,
+                                                                         const uint32_t* queue,
+                                                                         const uint32_t* count,
                                                                          uint32_t* cursor, uint32_t* medQueue,
-                                                                         uint32_t* medCount) {
-    waveBegin(true);
+                                                                         uint32_t* medCount, const uint32_t* mark) {
+    waveBeginBeside(mark);
     const uint32_t n = *count;
 #if SLRGPU_TRACE_REFILL
     if (n == 0) {
@@ -1354,7 +1391,7 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadowVol(DevSc
     }
 #endif
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ws.stats[1], (unsigned long long)n);
-    waveEnd(true);
+    waveEndBeside();
 }
 
 // Medium transmittance of the unoccluded shadow rays: one ratio-tracking walk
@@ -1367,12 +1404,13 @@ __global__ void __launch_bounds__(256, SLRGPU_TRACE_MIN_BLOCKS) kShadowVol(DevSc
 #define SLRGPU_MEDIUM_MIN_BLOCKS 4     // 64 registers; measured best of 2, 3, 4
 #endif
 __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kShadowVolMedium(DevScene sc, WaveState ws,
-                                                                                  const uint32_t* __restrict__ queue,
-                                 const uint32_t* __restrict__ count, uint32_t* take, uint32_t bounce) {
-    waveBegin(true);
+                                                                                  const uint32_t* queue,
+                                 const uint32_t* count, uint32_t* take, uint32_t bounce,
+                                 const uint32_t* mark) {
+    waveBeginBeside(mark);
     const uint32_t n = *count * kNumLambda;
     if (n == 0) {
-        waveEnd(true);
+        waveEndBeside();
         return;
     }
     trRun(
@@ -1398,7 +1436,7 @@ __global__ void __launch_bounds__(256, SLRGPU_MEDIUM_MIN_BLOCKS) kShadowVolMediu
             const size_t k = (size_t)queue[item / kNumLambda] * kNumLambda + item % kNumLambda;
             ws.L[k] += q.T * ws.shContrib[k];
         });
-    waveEnd(true);
+    waveEndBeside();
 }
 
 // Adds the wave's paths to the film: C = L * weight, dropped when not finite
@@ -1487,7 +1525,7 @@ __device__ __forceinline__ void filmStore(const WaveSegment &sg, uint32_t pix, u
 
 __global__ void __launch_bounds__(256, 3) kAccumulate(WaveState ws, const __grid_constant__ WaveParams wpArg,
                                                       const WaveParams* __restrict__ wpDev, uint32_t flags, float* out) {
-    waveBegin(false);
+    waveBeginAfter(nullptr);
     const WaveParams &wp = wpDev ? *wpDev : wpArg;
     const uint32_t lane = threadIdx.x & (kFilmLanes - 1), bin0 = lane * kFilmBins;
     const uint32_t quad = 0xfu << (threadIdx.x & 28);
@@ -2235,7 +2273,7 @@ static void surfaceBounce(const DevScene &sc, const DevScene* scenes, uint32_t k
         uint32_t* last = ctr - kCtrStride;
         lm.begin(SLRGPU_KERNEL_SHADOW);
         launchWaveKernel(kShadow<MULTI>, MULTI ? g.shadowM : g.shadow, stream, sc, w, w.shadowQueue, last + kCtrShadow,
-                         last + kCtrShadowTake, scenes);
+                         last + kCtrShadowTake, ctr + kCtrExtMark, scenes);
         lm.end();
         ++launches;
     }
@@ -2243,7 +2281,7 @@ static void surfaceBounce(const DevScene &sc, const DevScene* scenes, uint32_t k
     if (env) {
         lm.begin(SLRGPU_KERNEL_SHADE);
         launchWaveKernel(kShadeMiss<MULTI>, MULTI ? g.shadeMissM : g.shadeMiss, stream, sc, w,
-                         w.classQueue + (size_t)kClassMiss * w.N, ctr + kClassMiss, scenes, beside);
+                         w.classQueue + (size_t)kClassMiss * w.N, ctr + kClassMiss, scenes, ctr + kCtrShadeMark, beside);
         lm.end();
         ++launches;
         beside = true;
@@ -2262,7 +2300,7 @@ static void surfaceBounce(const DevScene &sc, const DevScene* scenes, uint32_t k
         lm.begin(SLRGPU_KERNEL_SHADE);
 #define SLRGPU_SHADESURF(KK)                                                                                  \
     launchWaveKernel(kShadeSurf<KK, MULTI>, grid, stream, sc, w, D, cq, ctr + k, outQueue, next + kCtrExt, \
-                     w.shadowQueue, ctr + kCtrShadow, scenes, beside)
+                     w.shadowQueue, ctr + kCtrShadow, scenes, ctr + kCtrShadeMark, beside)
         switch (k) {
         case kMatMatte: SLRGPU_SHADESURF(kMatMatte); break;
         case kMatSpecularReflection: SLRGPU_SHADESURF(kMatSpecularReflection); break;
@@ -2298,7 +2336,7 @@ static void volumetricBounce(const DevScene &sc, uint32_t kindMask, const WaveSt
     if (last) {
         lm.begin(SLRGPU_KERNEL_SHADOW);
         launchWaveKernel(kShadowVol, g.shadowVol, stream, sc, w, w.shadowQueue, last + kCtrShadow,
-                         last + kCtrShadowTake, medQueue, last + kCtrMedShadow);
+                         last + kCtrShadowTake, medQueue, last + kCtrMedShadow, ctr + kCtrExtMark);
         lm.end();
         ++launches;
     }
@@ -2309,7 +2347,7 @@ static void volumetricBounce(const DevScene &sc, uint32_t kindMask, const WaveSt
     if (last) {
         lm.begin(SLRGPU_KERNEL_SHADOW);
         launchWaveKernel(kShadowVolMedium, g.shadowVolMedium, stream, sc, w, medQueue, last + kCtrMedShadow,
-                         last + kCtrMedTake, b - 1);
+                         last + kCtrMedTake, b - 1, ctr + kCtrVolMark);
         lm.end();
         ++launches;
     }
@@ -2322,7 +2360,7 @@ static void volumetricBounce(const DevScene &sc, uint32_t kindMask, const WaveSt
         lm.begin(SLRGPU_KERNEL_SHADE);
 #define SLRGPU_SHADEVOL(KK)                                                                                      \
     launchWaveKernel(kShadeVol<KK>, g.shadeVol[KK], stream, sc, w, D, cq, ctr + k, outQueue, next + kCtrExt, \
-                     w.shadowQueue, ctr + kCtrShadow, beside)
+                     w.shadowQueue, ctr + kCtrShadow, ctr + kCtrShadeMark, beside)
         switch (k) {
         case 0: SLRGPU_SHADEVOL(0); break;
         case 1: SLRGPU_SHADEVOL(1); break;
