@@ -903,11 +903,15 @@ __global__ void __launch_bounds__(256, K == kMatGGXScattering ? SLRGPU_SHADE_DIE
 // The counters of the bounces keep their meaning: every ray, class and shadow
 // ray is counted in the row of its bounce.
 //
-// Scenes with a smooth dielectric keep to the bounce kernels: compiled here,
-// its refracted direction differs in the last bit, and glass that stands on a
-// surface turns that into another path.  (The other kinds' paths are the
-// same: on the terrain of 176k triangles and the box no ray count changed with
-// every bounce below 131072 paths in this kernel.)
+// Which kernel shades a vertex depends on how many paths its wave has left, and
+// so on the split into waves, which no film may show (films resumed over sample
+// ranges and served films equal slrgpu_render's bit for bit).  The kernel
+// therefore takes only scenes of the kinds that come out of it with the same
+// bits as out of the bounce kernels (kTailKinds; checked for each of them by
+// rendering the same paths both ways).  The dielectrics do not: compiled here,
+// the smooth one's refracted direction and the rough one's throughput differ
+// in the last bit, now and then into another path.  Their scenes keep to the
+// bounce kernels.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void countRows(uint32_t* counters, uint32_t row, uint32_t column, bool pred) {
     // lanes of a warp are at the same bounce unless some took a new path
@@ -922,6 +926,7 @@ __device__ __forceinline__ void countRows(uint32_t* counters, uint32_t row, uint
     }
 }
 
+constexpr uint32_t kTailKinds = 1u << kMatMatte | 1u << kMatSpecularReflection | 1u << kMatGGXReflection;
 template <bool MULTI>
 __global__ void __launch_bounds__(256, 1) kTail(DevScene scArg, WaveState ws, uint32_t maxDepth,
                                                                    const DevScene* __restrict__ scenes) {
@@ -978,7 +983,6 @@ __global__ void __launch_bounds__(256, 1) kTail(DevScene scArg, WaveState ws, ui
         SLRGPU_TAIL_CLASS(kMatMatte)
         SLRGPU_TAIL_CLASS(kMatSpecularReflection)
         SLRGPU_TAIL_CLASS(kMatGGXReflection)
-        SLRGPU_TAIL_CLASS(kMatGGXScattering)
 #undef SLRGPU_TAIL_CLASS
         if (__any_sync(0xffffffffu, cls == kClassMiss)) {
             countRows(ws.counters, row, kClassMiss, cls == kClassMiss);
@@ -2398,7 +2402,7 @@ static int runWave(const DeviceScene &ds0, const WaveState &w0, const WaveParams
     ds.sc.rngTape = rngTape;
     const WaveGrids &g = waveGrids(256);
     const uint32_t kinds = multi ? multi->kindMask : ds.kindMask;
-    const uint32_t tailPaths = volumetric || (kinds >> kMatSpecularScattering & 1u) ? 0u : SLRGPU_TAIL_PATHS;
+    const uint32_t tailPaths = volumetric || (kinds & ~kTailKinds) ? 0u : SLRGPU_TAIL_PATHS;
     const WaveStream order{stream, wpDev == nullptr && multi == nullptr};
     uint64_t launches = 0;
     CUDA_TRY(cudaMemsetAsync(w0.counters, 0, (size_t)kCtrStride * (D + 2) * sizeof(uint32_t), stream));
