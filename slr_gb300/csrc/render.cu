@@ -7,6 +7,7 @@
 // added to the 16-bin film with compensated summation.  The estimator is the
 // reference's PTRenderer::Job::contribution (libSLR/Renderer/PTRenderer.cpp:146-276)
 // and Job::kernel (:103-144); only the random numbers differ (counter-based).
+#include "ray_blocks.h"
 #include "render_api.h"
 #include "trace_ranges.h"
 
@@ -1647,10 +1648,9 @@ __device__ __forceinline__ void traceQueries(const DevScene &sc, const float4* _
                                              uint32_t* prim, float* t, float* b1, float* b2, StackEntry* shared,
                                              uint32_t* cursor) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t chunk = ((uint64_t)n + gridDim.x - 1) / gridDim.x;
-    const uint64_t first = (uint64_t)blockIdx.x * chunk;
-    const uint32_t end = first + chunk < n ? (uint32_t)(first + chunk) : n;
-    if (threadIdx.x == 0) *cursor = first < n ? (uint32_t)first : n;
+    const uint64_t chunk = raysPerBlock(n, gridDim.x);
+    const RayBlock own = rayBlock(n, gridDim.x, blockIdx.x);
+    if (threadIdx.x == 0) *cursor = 0;
     __syncthreads();
     const uint32_t width = (uint32_t)min((chunk + 7) / 8, (uint64_t)32);
     const uint32_t refill = min(width, (uint32_t)SLRGPU_QUERY_REFILL_LANES);
@@ -1670,11 +1670,11 @@ __device__ __forceinline__ void traceQueries(const DevScene &sc, const float4* _
             uint32_t base = 0;
             if ((int)lane == leader) base = atomicAdd(cursor, (uint32_t)__popc(idle));
             base = __shfl_sync(0xffffffffu, base, leader);
-            drained = base >= end || end - base <= (uint32_t)__popc(idle);
+            drained = raysDrained(base, (uint32_t)__popc(idle), own.count);
             if ((idle >> lane) & 1u) {
                 const uint32_t k = base + (uint32_t)__popc(idle & ((1u << lane) - 1));
-                if (base < end && k < end) {
-                    i = k;
+                if (k < own.count) {
+                    i = own.first + k;
                     const float4 o = rays[2 * (size_t)i], d = rays[2 * (size_t)i + 1];
                     const V3 org = V3{o.x, o.y, o.z}, dir = V3{d.x, d.y, d.z};
                     fin = ANY ? aw.begin(sc, org, dir, o.w, d.w) : cw.begin(sc, org, dir, o.w, d.w);
