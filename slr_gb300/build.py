@@ -22,7 +22,7 @@ LIB_DIR = PKG / "lib"
 LIB = LIB_DIR / "libslrgpu.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-HOST_SOURCES = ["scene_host.cpp", "capi.cpp", "server.cpp"]
+HOST_SOURCES = ["scene_host.cpp", "capi.cpp", "server.cpp", "bounce_counts.cpp"]
 CUDA_SOURCES = ["render.cu", "bpt.cu"]
 
 

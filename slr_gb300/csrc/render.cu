@@ -2017,53 +2017,6 @@ int RenderEngine::queueCounts(uint32_t* out, uint32_t capacity, uint32_t* rows) 
     return SLRGPU_OK;
 }
 
-int BounceCounts::begin(uint32_t bounces) {
-    if (bounces > capacity) {
-        release();
-        const cudaError_t e = cudaMallocHost(&host, bounces * sizeof(*host));
-        if (e != cudaSuccess) {
-            host = nullptr;
-            setError(std::string("bounce counts: ") + cudaGetErrorString(e));
-            return SLRGPU_ERR_OUT_OF_MEMORY;
-        }
-        capacity = bounces;
-        std::memset(host, 0, bounces * sizeof(*host));
-        tag = 0;
-    }
-    ++tag;   // the waves of 2^32 before it are long complete
-    if (tag == 0) tag = 1;
-    return SLRGPU_OK;
-}
-
-cudaError_t BounceCounts::get(uint32_t bounce, cudaStream_t stream, uint32_t* count) {
-    const volatile unsigned long long* word = host + bounce;
-    for (uint32_t spins = 1;; ++spins) {
-        unsigned long long v = *word;
-        if ((uint32_t)(v >> 32) == tag) {
-            *count = (uint32_t)v;
-            return cudaSuccess;
-        }
-        if ((spins & 0xfff) == 0) {
-            // a stream that has run dry has written the word, or failed
-            const cudaError_t e = cudaStreamQuery(stream);
-            if (e == cudaErrorNotReady) {
-                // not an error: leave no trace for the check after the wave
-                if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();
-                continue;
-            }
-            v = *word;
-            *count = (uint32_t)v;
-            return e != cudaSuccess ? e : ((uint32_t)(v >> 32) == tag ? cudaSuccess : cudaErrorUnknown);
-        }
-    }
-}
-
-void BounceCounts::release() {
-    if (host) cudaFreeHost(host);
-    host = nullptr;
-    capacity = 0;
-}
-
 int RenderEngine::ensureFilm(uint32_t P) {
     if (filmPixels >= P) return SLRGPU_OK;
     if (filmSum) cudaFree(filmSum);
@@ -2413,7 +2366,7 @@ static int runWave(const DeviceScene &ds0, const WaveState &w0, const WaveParams
     WaveState w = w0;
     w.hostCounts = nullptr;
     if (counts) {
-        if (int rc = counts->begin(D + 1)) return rc;
+        if (int rc = counts->begin(D + 1, stream)) return rc;
         w.hostCounts = counts->host;
         w.hostTag = counts->tag;
     }

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../../include/slrgpu.h"
+#include "bounce_counts.h"
 #include "scene_host.h"
 #include "slrgpu_types.h"
 
@@ -38,18 +39,6 @@ inline uint64_t deviceSceneBytes(const DeviceScene &ds) {
 
 struct WaveState;
 struct BptEngine;   // bidirectional path state (bpt.cu)
-
-// The number of paths that start each bounce of a wave, which the bounce's
-// first kernel writes to pinned host memory together with the wave's tag.
-struct BounceCounts {
-    unsigned long long* host = nullptr;   // [capacity], pinned
-    uint32_t capacity = 0;
-    uint32_t tag = 0;
-    int begin(uint32_t bounces);   // a new wave
-    // waits until the bounce has started; an error of the stream ends the wait
-    cudaError_t get(uint32_t bounce, cudaStream_t stream, uint32_t* count);
-    void release();
-};
 
 // Per-context path state and film buffers, grown on demand.
 struct RenderEngine {
