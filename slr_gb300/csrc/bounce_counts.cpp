@@ -1,5 +1,8 @@
 #include "bounce_counts.h"
 
+#include <sched.h>
+#include <time.h>
+
 #include <cstring>
 #include <string>
 
@@ -24,6 +27,8 @@ int BounceCounts::begin(uint32_t bounces, cudaStream_t stream) {
         std::memset(host, 0, bounces * sizeof(*host));
         tag = 0;
     }
+    unsigned int flags = 0;
+    schedule = cudaGetDeviceFlags(&flags) == cudaSuccess ? flags & cudaDeviceScheduleMask : 0;
     ++tag;   // the waves of 2^32 before it are long complete
     if (tag == 0) tag = 1;
     return SLRGPU_OK;
@@ -31,20 +36,32 @@ int BounceCounts::begin(uint32_t bounces, cudaStream_t stream) {
 
 cudaError_t BounceCounts::get(uint32_t bounce, cudaStream_t stream, uint32_t* count) {
     const volatile unsigned long long* word = host + bounce;
+    // A device set to let its waiting threads sleep or yield has them do so
+    // here too, as cudaStreamSynchronize would; the next bounce is launched
+    // already, so a late look costs the GPU nothing.
+    const bool spin = schedule != cudaDeviceScheduleBlockingSync && schedule != cudaDeviceScheduleYield;
     for (uint32_t looks = 1;; ++looks) {
         unsigned long long v = *word;
         if ((uint32_t)(v >> 32) == tag) {
             *count = (uint32_t)v;
             return cudaSuccess;
         }
-        if ((looks & 0xfff) != 0) continue;
+        if (spin && (looks & 0xfff) != 0) continue;
         // a kernel of the wave that was refused at its launch never writes
         const cudaError_t pending = cudaGetLastError();
         if (pending != cudaSuccess && pending != cudaErrorNotReady) return pending;
         // a stream that has run dry has written the word, or failed
         const cudaError_t e = cudaStreamQuery(stream);
         if (e != cudaSuccess) cudaGetLastError();   // "not ready" is no error: no trace for the check after the wave
-        if (e == cudaErrorNotReady) continue;
+        if (e == cudaErrorNotReady) {
+            if (schedule == cudaDeviceScheduleBlockingSync) {
+                const timespec nap = {0, 50000};
+                nanosleep(&nap, nullptr);
+            } else if (schedule == cudaDeviceScheduleYield) {
+                sched_yield();
+            }
+            continue;
+        }
         v = *word;
         *count = (uint32_t)v;
         if (e != cudaSuccess) return e;

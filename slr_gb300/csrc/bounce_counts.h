@@ -13,6 +13,7 @@ struct BounceCounts {
     unsigned long long* host = nullptr;   // [capacity], pinned
     uint32_t capacity = 0;
     uint32_t tag = 0;
+    uint32_t schedule = 0;                // how the device's host threads wait (cudaDeviceSchedule*)
 
     // A new wave on the stream.  On failure, an error code of the C ABI.
     int begin(uint32_t bounces, cudaStream_t stream);

@@ -2,6 +2,7 @@
  * runtime made of the few calls it needs, whose answers each case scripts. */
 #include <cstdio>
 #include <cstdlib>
+#include <ctime>
 #include <functional>
 #include <string>
 #include <vector>
@@ -10,6 +11,7 @@
 
 static cudaError_t g_last = cudaSuccess;          // the thread's pending error
 static std::function<cudaError_t()> g_query;      // the stream's state
+static unsigned int g_flags = 0;
 static int g_queries = 0;
 static std::vector<std::string> g_calls;
 
@@ -18,6 +20,7 @@ cudaError_t cudaMallocHost(void** p, size_t n) { *p = std::malloc(n); return cud
 cudaError_t cudaFreeHost(void* p) { g_calls.push_back("free"); std::free(p); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { g_calls.push_back("synchronize"); return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "error"; }
+cudaError_t cudaGetDeviceFlags(unsigned int* f) { *f = g_flags; return cudaSuccess; }
 cudaError_t cudaGetLastError() { cudaError_t e = g_last; g_last = cudaSuccess; return e; }
 cudaError_t cudaPeekAtLastError() { return g_last; }
 cudaError_t cudaStreamQuery(cudaStream_t) {
@@ -74,6 +77,21 @@ int main() {
     CHECK(c.begin(20, nullptr) == 0 && c.capacity == 20);
     CHECK((g_calls == std::vector<std::string>{"synchronize", "free"}));
 
+    // Waiting threads of the device sleep: the wait for a bounce that takes 0.2 s costs next to no processor time.
+    for (unsigned int flags : {(unsigned int)cudaDeviceScheduleBlockingSync, (unsigned int)cudaDeviceScheduleYield}) {
+        g_flags = flags | cudaDeviceMapHost;
+        fresh();
+        timespec t0, t1;
+        clock_gettime(CLOCK_MONOTONIC, &t0);
+        const std::clock_t cpu = std::clock();
+        g_query = [&]() {
+            clock_gettime(CLOCK_MONOTONIC, &t1);
+            if ((t1.tv_sec - t0.tv_sec) + 1e-9 * (t1.tv_nsec - t0.tv_nsec) > 0.2) c.host[2] = word(c.tag, 4);
+            return cudaErrorNotReady;
+        };
+        CHECK(c.get(2, nullptr, &n) == cudaSuccess && n == 4);
+        if (flags == cudaDeviceScheduleBlockingSync) CHECK((double)(std::clock() - cpu) / CLOCKS_PER_SEC < 0.1);
+    }
     c.release();
     std::printf("bad %d\n", g_bad);
     return g_bad != 0;
