@@ -1,7 +1,6 @@
 #include "bounce_counts.h"
 
 #include <sched.h>
-#include <time.h>
 
 #include <cstring>
 #include <string>
@@ -11,6 +10,11 @@
 namespace slrgpu {
 
 void setError(const std::string &msg);
+
+bool BounceCounts::wanted() {
+    unsigned int flags = 0;
+    return cudaGetDeviceFlags(&flags) != cudaSuccess || (flags & cudaDeviceScheduleMask) != cudaDeviceScheduleBlockingSync;
+}
 
 int BounceCounts::begin(uint32_t bounces, cudaStream_t stream) {
     if (bounces > capacity) {
@@ -27,8 +31,6 @@ int BounceCounts::begin(uint32_t bounces, cudaStream_t stream) {
         std::memset(host, 0, bounces * sizeof(*host));
         tag = 0;
     }
-    unsigned int flags = 0;
-    schedule = cudaGetDeviceFlags(&flags) == cudaSuccess ? flags & cudaDeviceScheduleMask : 0;
     ++tag;   // the waves of 2^32 before it are long complete
     if (tag == 0) tag = 1;
     return SLRGPU_OK;
@@ -36,17 +38,17 @@ int BounceCounts::begin(uint32_t bounces, cudaStream_t stream) {
 
 cudaError_t BounceCounts::get(uint32_t bounce, cudaStream_t stream, uint32_t* count) {
     const volatile unsigned long long* word = host + bounce;
-    // A device set to let its waiting threads sleep or yield has them do so
-    // here too, as cudaStreamSynchronize would; the next bounce is launched
-    // already, so a late look costs the GPU nothing.
-    const bool spin = schedule != cudaDeviceScheduleBlockingSync && schedule != cudaDeviceScheduleYield;
+    // as cudaStreamSynchronize would wait
+    unsigned int flags = 0;
+    const bool yield = cudaGetDeviceFlags(&flags) == cudaSuccess &&
+                       (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleYield;
     for (uint32_t looks = 1;; ++looks) {
         unsigned long long v = *word;
         if ((uint32_t)(v >> 32) == tag) {
             *count = (uint32_t)v;
             return cudaSuccess;
         }
-        if (spin && (looks & 0xfff) != 0) continue;
+        if (!yield && (looks & 0xfff) != 0) continue;
         // a kernel of the wave that was refused at its launch never writes
         const cudaError_t pending = cudaGetLastError();
         if (pending != cudaSuccess && pending != cudaErrorNotReady) return pending;
@@ -54,12 +56,7 @@ cudaError_t BounceCounts::get(uint32_t bounce, cudaStream_t stream, uint32_t* co
         const cudaError_t e = cudaStreamQuery(stream);
         if (e != cudaSuccess) cudaGetLastError();   // "not ready" is no error: no trace for the check after the wave
         if (e == cudaErrorNotReady) {
-            if (schedule == cudaDeviceScheduleBlockingSync) {
-                const timespec nap = {0, 50000};
-                nanosleep(&nap, nullptr);
-            } else if (schedule == cudaDeviceScheduleYield) {
-                sched_yield();
-            }
+            if (yield) sched_yield();
             continue;
         }
         v = *word;

@@ -13,8 +13,10 @@ struct BounceCounts {
     unsigned long long* host = nullptr;   // [capacity], pinned
     uint32_t capacity = 0;
     uint32_t tag = 0;
-    uint32_t schedule = 0;                // how the device's host threads wait (cudaDeviceSchedule*)
 
+    // Whether the host looks at all: it would wait awake, so not where the
+    // device's waiting threads are set to sleep (cudaDeviceScheduleBlockingSync).
+    static bool wanted();
     // A new wave on the stream.  On failure, an error code of the C ABI.
     int begin(uint32_t bounces, cudaStream_t stream);
     // Waits until the bounce has started.  An error that is pending when the

@@ -2365,6 +2365,7 @@ static int runWave(const DeviceScene &ds0, const WaveState &w0, const WaveParams
     }
     WaveState w = w0;
     w.hostCounts = nullptr;
+    if (counts && !BounceCounts::wanted()) counts = nullptr;
     if (counts) {
         if (int rc = counts->begin(D + 1, stream)) return rc;
         w.hostCounts = counts->host;
@@ -2381,7 +2382,8 @@ static int runWave(const DeviceScene &ds0, const WaveState &w0, const WaveParams
     // one launches them until it sees (one bounce late, so that the GPU never
     // waits for the host) that a bounce has no paths or was left to the tail
     // kernel, or, where the host may not look (graph capture, the
-    // asynchronous entry point), for every bounce.
+    // asynchronous entry point, a device whose waiting threads sleep), for
+    // every bounce.
     const bool tailOnly = !volumetric && wpDev == nullptr && wp.numPaths <= tailPaths;
     for (uint32_t b = 0; b <= D && !tailOnly; ++b) {
         if (counts && b >= 2) {

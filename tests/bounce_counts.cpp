@@ -2,7 +2,6 @@
  * runtime made of the few calls it needs, whose answers each case scripts. */
 #include <cstdio>
 #include <cstdlib>
-#include <ctime>
 #include <functional>
 #include <string>
 #include <vector>
@@ -77,21 +76,16 @@ int main() {
     CHECK(c.begin(20, nullptr) == 0 && c.capacity == 20);
     CHECK((g_calls == std::vector<std::string>{"synchronize", "free"}));
 
-    // Waiting threads of the device sleep: the wait for a bounce that takes 0.2 s costs next to no processor time.
-    for (unsigned int flags : {(unsigned int)cudaDeviceScheduleBlockingSync, (unsigned int)cudaDeviceScheduleYield}) {
+    // Where waiting threads are set to sleep the host does not look; where they yield it looks every time.
+    for (unsigned int flags : {0u, (unsigned int)cudaDeviceScheduleSpin, (unsigned int)cudaDeviceScheduleYield}) {
         g_flags = flags | cudaDeviceMapHost;
+        CHECK(BounceCounts::wanted());
         fresh();
-        timespec t0, t1;
-        clock_gettime(CLOCK_MONOTONIC, &t0);
-        const std::clock_t cpu = std::clock();
-        g_query = [&]() {
-            clock_gettime(CLOCK_MONOTONIC, &t1);
-            if ((t1.tv_sec - t0.tv_sec) + 1e-9 * (t1.tv_nsec - t0.tv_nsec) > 0.2) c.host[2] = word(c.tag, 4);
-            return cudaErrorNotReady;
-        };
-        CHECK(c.get(2, nullptr, &n) == cudaSuccess && n == 4);
-        if (flags == cudaDeviceScheduleBlockingSync) CHECK((double)(std::clock() - cpu) / CLOCKS_PER_SEC < 0.1);
+        g_query = [&]() { if (g_queries == 3) c.host[2] = word(c.tag, 4); return cudaErrorNotReady; };
+        CHECK(c.get(2, nullptr, &n) == cudaSuccess && n == 4 && g_queries == 3 && g_last == cudaSuccess);
     }
+    g_flags = cudaDeviceScheduleBlockingSync | cudaDeviceMapHost;
+    CHECK(!BounceCounts::wanted());
     c.release();
     std::printf("bad %d\n", g_bad);
     return g_bad != 0;

@@ -1,7 +1,7 @@
 """The host's wait for the sizes of a wave's bounces, on the host against a
 scripted CUDA runtime: which counts it takes, that the cause of a refused launch
 is what it returns and that no error stays pending, that a stream which has run
-dry ends it, and that it sleeps on devices whose waiting threads do."""
+dry ends it, and that there is none on devices whose waiting threads sleep."""
 import shutil
 import subprocess
 from pathlib import Path
