@@ -180,12 +180,23 @@ REFERENCE_BUILD_FLAGS = ("the reference renderer built from its own sources with
                   "default floating-point contraction) and build-only patches P1-P4, P6-P11 (oracle/build_ref.py)")
 
 
+def reference_missing():
+    """Why the reference renderer cannot run here, or None."""
+    from oracle import oracle as O
+    if O.TIMING_LIB_PATH.is_file():
+        return None
+    return f"the reference renderer is not built here ({O.TIMING_LIB_PATH.name} is missing; its sources are needed)"
+
+
 def cpu_baseline(desc, threads: int, seconds_cap: float = 40.0):
     """The reference renderer on the workload's own frame: the whole frame
     (all spp) when one pass predicts it within seconds_cap, else as many
     whole passes as fit.  The reference renders a frame as spp passes of one
     sample per pixel over all tiles (PTRenderer.cpp:65-75), so passes are its
     unit of work."""
+    why = reference_missing()
+    if why:
+        return {"unavailable": why}
     from oracle import oracle as O
     O.use_timing_build()
     t0 = time.time()
@@ -485,6 +496,10 @@ def main():
         if args.workload in ("serving", "traversal"):
             print(json.dumps({"impl": "reference", "unavailable": "the reference has no serving loop; its "
                               "traversal is timed by --workload traversal's cpu_baseline"}))
+            return 0
+        if reference_missing():
+            if int(os.environ.get("RANK", "0")) == 0:
+                print(json.dumps({"impl": "reference", "unavailable": reference_missing()}))
             return 0
         return run_reference(args)
 
