@@ -2767,12 +2767,44 @@ __global__ void __launch_bounds__(256) kFilmToBmp(const float* __restrict__ film
     }
 }
 
+// Device memory for the films of small images, in the library's image on each GPU.
+// What an allocation costs depends on what the driver has in hand: a block
+// that it can cut from memory of its own is a few us, one that it has to map, and
+// unmap again, a hundred, and where the line lies changes with whatever else
+// the process holds (736 x 44, a film of 2.07 MB behind other work: 87 us by two
+// blocks, 190 by one, in another process 63 and 185).  One call at a
+// time has the array; others, and larger films, whose blocks are mapped in any
+// case, allocate.
+constexpr size_t kFilmScratchBytes = (2u << 20) + (256u << 10);
+static __device__ __align__(256) unsigned char g_filmScratch[kFilmScratchBytes];
+
+// The array on the current device while `hold` has its lock, or null.
+static uint8_t* filmScratch(std::unique_lock<std::mutex> &hold) {
+    constexpr int kDevices = 64;
+    static std::mutex mu[kDevices];
+    static uint8_t* address[kDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return nullptr;
+    std::unique_lock<std::mutex> lock(mu[dev], std::try_to_lock);
+    if (!lock) return nullptr;
+    if (!address[dev]) {
+        void* p = nullptr;
+        if (cudaGetSymbolAddress(&p, g_filmScratch) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        address[dev] = (uint8_t*)p;
+    }
+    hold = std::move(lock);
+    return address[dev];
+}
+
 // Takes the page faults of a caller's array here, on the host, leaving its bytes
 // as they are: a copy from the device into pages that nobody has touched has
-// them one at a time behind the copy, which made the rows of small films in new
-// arrays slower than a copy by way of a vector (33 x 33: 222 us by the vector,
-// 272 straight into new pages, 208 so; 200 x 150: 247, 309, 227; 1920 x 1080:
-// 1725, 1369, 1262).  The step is the smallest page size of the hosts.
+// them one at a time behind the copy, which made the rows of films in new arrays
+// slower than a copy by way of a vector (400 x 300: 315 us by the vector, 409
+// straight into new pages, 280 so; 1920 x 1080: 1725, 1369, 1262).  The step is
+// the smallest page size of the hosts.
 static void touchPages(uint8_t* p, size_t bytes) {
     volatile uint8_t* q = p;
     for (size_t at = 0; at < bytes; at += 4096) q[at] = q[at];
@@ -2797,8 +2829,9 @@ int filmToBmp(const float* film, uint32_t width, uint32_t height, bool filmOnDev
     // tables: 0.2 ms faster for a buffer it has read before, 3.2 ms slower for
     // a 1920 x 1080 film in new pages, whose translations come one by one.)
     const size_t copyBytes = filmOnDevice ? 0 : (filmBytes + 255) / 256 * 256;
-    uint8_t* buffer = nullptr;
-    cudaError_t e = cudaMalloc(&buffer, copyBytes + outBytes);
+    std::unique_lock<std::mutex> scratch;
+    uint8_t* buffer = copyBytes + outBytes <= kFilmScratchBytes ? filmScratch(scratch) : nullptr;
+    cudaError_t e = buffer ? cudaSuccess : cudaMalloc(&buffer, copyBytes + outBytes);
     if (e == cudaSuccess && !filmOnDevice) e = cudaMemcpy(buffer, film, filmBytes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         const float* src = filmOnDevice ? film : (const float*)buffer;
@@ -2811,7 +2844,7 @@ int filmToBmp(const float* film, uint32_t width, uint32_t height, bool filmOnDev
         touchPages(pixels, outBytes);   // while the kernel runs
     }
     if (e == cudaSuccess) e = cudaMemcpy(pixels, buffer + copyBytes, outBytes, cudaMemcpyDeviceToHost);
-    if (buffer) cudaFree(buffer);
+    if (buffer && !scratch) cudaFree(buffer);
     if (e != cudaSuccess) {
         setError(cudaGetErrorString(e));
         return SLRGPU_ERR_CUDA;
