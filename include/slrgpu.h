@@ -81,7 +81,9 @@ typedef struct slrgpu_settings {
 } slrgpu_settings;
 
 /* settings.flags: record CUDA events around every launch and report the
- * device time per kernel class in slrgpu_render_stats.kernel_ms. */
+ * device time per kernel class in slrgpu_render_stats.kernel_ms.  The events
+ * keep apart kernels that otherwise overlap, so such a frame takes longer than
+ * one without the flag, most of all a small one. */
 #define SLRGPU_FLAG_PROFILE_KERNELS 1u
 /* settings.flags: watertight ray-triangle test (Woop, Benthin, Wald 2013)
  * instead of the reference's Moller-Trumbore order, which can let a ray

@@ -173,10 +173,9 @@ struct SharedStack {
 // three 32-byte halves of its box planes and its child words instead of seven
 // 16-byte parts, testing two boxes per packed instruction and ordering the
 // children without carrying their numbers took 1,000,003 incoherent closest-hit
-// queries on 24k triangles from 489 to 456 us, 4 Mi any-hit queries on 176k
-// triangles from 1697 to 1528 us and the 1,034,242-triangle frame from 66.9 to
-// 64.6 ms (without the loads 476 us, 1675 us and 65.2 ms, without the packed
-// tests 465 us, 1561 us and 66.3 ms).
+// queries on 24k triangles from 489 to 456 us and 4 Mi any-hit queries on 176k
+// triangles from 1697 to 1528 us (without the loads 476 and 1675 us, without the
+// packed tests 465 and 1561 us).
 
 // 32 bytes of read-only global memory in one load (p 32-byte aligned).
 __device__ __forceinline__ void ldg256(const float4* p, float4 &a, float4 &b) {

@@ -2248,7 +2248,9 @@ static void surfaceBounce(const DevScene &sc, const DevScene* scenes, uint32_t k
     // kinds' long kernels go first and the others run beside them (333 x 187 x 24
     // with every kind 2.04 to 1.94 ms, 176k-triangle terrain at 512 x 512 x 4 2.20
     // to 2.17 ms); a wave that fills the GPU in each of them loses half a
-    // percent that way (64 Mi paths of the 1M-triangle terrain).
+    // percent that way (64 Mi paths of the 1M-triangle terrain; nothing was
+    // measured between the two sizes).  A captured wave, whose size is not known
+    // at its capture, runs the kernels one after the other, in either order.
     const bool longFirst = numPaths <= kLongFirstPaths;
     for (int i = 0; i < kNumShadeClasses - 1; ++i) {
         const int k = longFirst ? kNumShadeClasses - 2 - i : i;
@@ -2336,11 +2338,18 @@ static void volumetricBounce(const DevScene &sc, uint32_t kindMask, const WaveSt
 }
 
 // Bounces of the surface path tracer that start with at most this many
-// paths go to kTail.  A 64 x 64 x 1 frame of the box (4096 paths): 392 us with
-// bounce kernels alone, 237 us in the tail kernel; the 176k-triangle terrain
-// at 512 x 512 x 4: 2458 us with bounce kernels alone, 2397 us at this line,
-// 2935 us with the line at 10000, where the tail's mixed warps cost more than
-// the bounces' launches.
+// paths go to kTail.  Frames in us with bounce kernels alone, with this line and
+// with one at 16384:
+//   box, matte                 64 x 64 x 1    389  222  222
+//                              72 x 64 x 1    413  240  211
+//                             128 x 96 x 1    450  284  224
+//                             200 x 160 x 2   511  396  367
+//                             256 x 256 x 16 1295 1304 1295
+//   42k triangles, conductors  72 x 64 x 1    441  299  233
+//                             128 x 128 x 1   539  393  345
+//                             256 x 256 x 4   979  747  746
+// (The higher line is the better one here; larger scenes of these kinds were
+// not measured with it.)
 #ifndef SLRGPU_TAIL_PATHS
 #define SLRGPU_TAIL_PATHS 4096u
 #endif
