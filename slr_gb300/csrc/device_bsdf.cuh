@@ -300,9 +300,16 @@ __device__ __forceinline__ void ggxTransmitPairs(const Bsdf &B, bool entering, V
 }
 
 // Visible-normal sampling (Heitz 2017, "A Simpler and Exact Sampling Routine
-// for the GGX Distribution of Visible Normals").
+// for the GGX Distribution of Visible Normals").  FUSED: the squared length of
+// the stretched direction with its multiply-adds written out.  The surface path
+// tracer's rough dielectric asks for it: left to the compiler, the sum came out
+// with other products fused in the bounce kernel (as written here) than in the
+// tail kernel, and films depended on which of the two shaded a vertex.
+template <bool FUSED = false>
 __device__ __forceinline__ float ggxSample(float ax, float ay, V3 v, float u0, float u1, V3* m, float* pdf) {
-    V3 sv = normalize(V3{ax * v.x, ay * v.y, v.z});
+    const V3 s = V3{ax * v.x, ay * v.y, v.z};
+    const float s2 = FUSED ? __fmaf_rn(s.z, s.z, __fmaf_rn(s.x, s.x, __fmul_rn(s.y, s.y))) : dot(s, s);
+    const V3 sv = s * (1.0f / sqrtf(s2));
     float dist2D = sqrtf(sv.x * sv.x + sv.y * sv.y);
     float rec = 1.0f / dist2D;
     V3 T1 = (sv.z < 0.9999f) ? V3{sv.y * rec, -sv.x * rec, 0} : V3{1, 0, 0};
@@ -333,7 +340,7 @@ __device__ __forceinline__ void specScale(const Spec &a, float s, Spec &out) {
 // shades a single material), K < 0 dispatches on B.kind at run time.
 
 // Returns fs (without the shading-normal correction); res->pdf == 0 on failure.
-template <int K>
+template <int K, bool FUSED = false>
 __device__ __forceinline__ void bsdfSampleBody(const Bsdf &B, const BsdfQuery &q, float uc, float u0, float u1,
                                                BsdfSample* res, Spec &fs) {
     res->pdf = 0.0f;
@@ -423,7 +430,7 @@ __device__ __forceinline__ void bsdfSampleBody(const Bsdf &B, const BsdfQuery &q
         float sign = entering ? 1.0f : -1.0f;
         V3 m;
         float mPdf;
-        float D = ggxSample(B.ax, B.ay, sign * q.dir, u0, u1, &m, &mPdf);
+        float D = ggxSample<FUSED>(B.ax, B.ay, sign * q.dir, u0, u1, &m, &mPdf);
         float dotHV = dot(q.dir, m);
         if (dotHV * sign <= 0 || isnan(D)) return;
         Spec F;
@@ -574,11 +581,12 @@ static __device__ __noinline__ float bsdfPdfInternal(const Bsdf &B, const BsdfQu
 
 // ---- the BSDF wrapper: shading-normal correction |d.z / dot(d, n_g)| ----
 // K < 0: any material (run-time dispatch); K >= 0: that material kind only.
-template <int K = -1>
+// FUSED: see ggxSample.
+template <int K = -1, bool FUSED = false>
 __device__ __forceinline__ void bsdfSample(const Bsdf &B, const BsdfQuery &q, float uc, float u0, float u1,
                                            BsdfSample* res, Spec &fs) {
     if (K < 0) bsdfSampleInternal(B, q, uc, u0, u1, res, fs);
-    else bsdfSampleBody<K>(B, q, uc, u0, u1, res, fs);
+    else bsdfSampleBody<K, FUSED>(B, q, uc, u0, u1, res, fs);
     if (res->pdf == 0.0f) return;
     float sn = fabsf(res->dir.z / dot(res->dir, q.gn));
 #pragma unroll

@@ -828,7 +828,7 @@ __device__ __forceinline__ void shadeVertex(const DevScene &scArg, const WaveSta
         float uc = rng.next(), u0 = rng.next(), u1 = rng.next();
         BsdfSample bs;
         Spec fs;
-        bsdfSample<K>(B, q, uc, u0, u1, &bs, fs);
+        bsdfSample<K, true>(B, q, uc, u0, u1, &bs, fs);
         if (bs.pdf == 0.0f || specIsZero(fs)) {
             alive = false;
         } else {
@@ -910,10 +910,9 @@ __global__ void __launch_bounds__(256, K == kMatGGXScattering ? SLRGPU_SHADE_DIE
 // ranges and served films equal slrgpu_render's bit for bit).  The kernel
 // therefore takes only scenes of the kinds that come out of it with the same
 // bits as out of the bounce kernels (kTailKinds; checked for each of them by
-// rendering the same paths both ways).  The dielectrics do not: compiled here,
-// the smooth one's refracted direction and the rough one's throughput differ
-// in the last bit, now and then into another path.  Their scenes keep to the
-// bounce kernels.
+// rendering the same paths both ways).  The smooth dielectric does not: compiled
+// here, its refracted direction differs in the last bit, and glass that stands on
+// a surface turns that into another path.  Its scenes keep to the bounce kernels.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void countRows(uint32_t* counters, uint32_t row, uint32_t column, bool pred) {
     // lanes of a warp are at the same bounce unless some took a new path
@@ -928,7 +927,8 @@ __device__ __forceinline__ void countRows(uint32_t* counters, uint32_t row, uint
     }
 }
 
-constexpr uint32_t kTailKinds = 1u << kMatMatte | 1u << kMatSpecularReflection | 1u << kMatGGXReflection;
+constexpr uint32_t kTailKinds = 1u << kMatMatte | 1u << kMatSpecularReflection | 1u << kMatGGXReflection |
+                                1u << kMatGGXScattering;
 template <bool MULTI>
 __global__ void __launch_bounds__(256, 1) kTail(DevScene scArg, WaveState ws, uint32_t maxDepth,
                                                                    const DevScene* __restrict__ scenes) {
@@ -985,6 +985,7 @@ __global__ void __launch_bounds__(256, 1) kTail(DevScene scArg, WaveState ws, ui
         SLRGPU_TAIL_CLASS(kMatMatte)
         SLRGPU_TAIL_CLASS(kMatSpecularReflection)
         SLRGPU_TAIL_CLASS(kMatGGXReflection)
+        SLRGPU_TAIL_CLASS(kMatGGXScattering)
 #undef SLRGPU_TAIL_CLASS
         if (__any_sync(0xffffffffu, cls == kClassMiss)) {
             countRows(ws.counters, row, kClassMiss, cls == kClassMiss);

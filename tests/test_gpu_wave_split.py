@@ -1,8 +1,8 @@
 """A film's bits do not depend on how its samples are split into waves, also
 where the split decides which kernels shade a bounce (waves of few paths are
 taken to their end by one kernel): every material kind alone among matte
-walls, and a height field of rough conductors and dielectrics under an
-environment, rendered whole, in waves of 4096 paths, of three samples and as
+walls, rough glass whose indices vary with the wavelength, and height fields of
+rough conductors and dielectrics under an environment, rendered whole, in waves of 4096 paths, of three samples and as
 a resumed film, and served beside larger requests."""
 import numpy as np
 import pytest
@@ -15,11 +15,19 @@ W, H, SPP, DEPTH = 64, 64, 16, 10
 
 
 def _desc(name):
+    if name == "dispersive":
+        d = _desc("microfacet_scattering")
+        outside = d.spectrum_regular(np.linspace(1.0, 1.02, 5).astype(np.float32), 360.0, 830.0)
+        inside = d.spectrum_regular(np.linspace(1.7, 1.45, 5).astype(np.float32), 360.0, 830.0)
+        glass = d.material("microfacet_scattering", (outside, inside), 0.1, 0.3)
+        d.materials = [d.materials[glass] if m.kind == "microfacet_scattering" else m for m in d.materials]
+        return d
     if name in KINDS:
         d = scenes.glossy_box_scene(W, H)
         d.materials = [m if m.kind in ("matte", "emitter", name) else d.materials[0] for m in d.materials]
         return d
-    d = scenes.heightfield_scene(grid=64, spheres=8, sphere_freq=6, env_size=(128, 64), width=W, height=H, seed=1)
+    d = scenes.heightfield_scene(grid=64, spheres=8, sphere_freq=6, env_size=(128, 64), width=W, height=H,
+                                 seed=int(name[7:] or 1) if name.startswith("terrain") else 1)
     if name == "conductors":
         matte = d.material("matte", (d.spectrum_rgb(REFLECTANCE, 0.7, 0.5, 0.3),))
         d.materials = [m if m.kind != "microfacet_scattering" else d.materials[matte] for m in d.materials]
@@ -27,7 +35,7 @@ def _desc(name):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("name", KINDS + ["conductors", "terrain"])
+@pytest.mark.parametrize("name", KINDS + ["dispersive", "conductors", "terrain0", "terrain1", "terrain2", "terrain3"])
 def test_film_does_not_depend_on_the_wave_split(name):
     scene = api.Scene(_desc(name))
     whole, st = scene.render(W, H, SPP, DEPTH, seed=5)
