@@ -2341,16 +2341,19 @@ static void volumetricBounce(const DevScene &sc, uint32_t kindMask, const WaveSt
 // Bounces of the surface path tracer that start with at most this many
 // paths go to kTail.  Frames in us with bounce kernels alone, with this line and
 // with one at 16384:
-//   box, matte                 64 x 64 x 1    389  222  222
-//                              72 x 64 x 1    413  240  211
-//                             128 x 96 x 1    450  284  224
-//                             200 x 160 x 2   511  396  367
-//                             256 x 256 x 16 1295 1304 1295
-//   42k triangles, conductors  72 x 64 x 1    441  299  233
-//                             128 x 128 x 1   539  393  345
-//                             256 x 256 x 4   979  747  746
-// (The higher line is the better one here; larger scenes of these kinds were
-// not measured with it.)
+//   box, matte                  64 x 64 x 1    389  222  222
+//                               72 x 64 x 1    413  240  211
+//                              128 x 96 x 1    450  284  224
+//                              200 x 160 x 2   511  396  367
+//                              256 x 256 x 16 1308 1314 1308
+//   42k triangles, conductors   72 x 64 x 1    441  299  233
+//                              128 x 128 x 1   543  386  345
+//                              256 x 256 x 4   979  747  746
+//   42k triangles, every rough  200 x 160 x 2 1054  679  685
+//   176k triangles, every rough 64 x 64 x 1    993  515  512
+//                              512 x 512 x 4  2184 2288 2642
+// A wave that starts with few paths gains from a higher line, the last bounces
+// of a large one lose.
 #ifndef SLRGPU_TAIL_PATHS
 #define SLRGPU_TAIL_PATHS 4096u
 #endif
