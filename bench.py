@@ -638,7 +638,7 @@ def main():
                             "compulsory 48 B (ray in, hit out)")
     if VOLUMETRIC and names[dom] == "shadow":
         roofline["note"] = ("the shadow class is dominated by the ratio-tracking transmittance walks, which read the "
-                            "density grid from L2 (64 MiB at 256^3; ~91 % L2 hit rate, ~73 % issue activity with 13 "
+                            "density grid from L2 (64 MiB at 256^3; ~84 % L2 hit rate, ~76 % issue activity with 16 "
                             "of 32 lanes active per instruction under ncu): issue- and latency-bound, not HBM-bound; "
                             "bytes_per_unit counts only the shadow ray's 36 B")
     if BPT:   # the bidirectional tracer's kernels behind the classes
