@@ -2203,7 +2203,8 @@ static void launchWaveKernel(void (*kernel)(P...), int grid, const WaveStream &w
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = ws.overlap ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);   // errors: cudaGetLastError after the wave
+    // an error stays pending: the wait for a bounce's count or the check after the wave returns it
+    cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);
 }
 
 constexpr uint32_t kLongFirstPaths = 4u << 20;
